@@ -192,7 +192,7 @@ int lbm_cu_deviation_stats(lbm_lattice *lat, double out[5], void *stream);
  * handed out under a budget, or a monitor that must not trigger the implicit
  * synchronisation of cudaMalloc/cudaFree, cannot afford that.  This variant
  * keeps its partial sums in a fixed device array inside the library
- * (1.3 MB, present on every GPU that loads the library until the process
+ * (160 KB, present on every GPU that loads the library until the process
  * exits) and calls no allocator.  Limit: lattices of at most 134,217,728
  * cells (512^3); larger ones are rejected with an error.  The first call on
  * a device looks up the array's device address, so make that first call

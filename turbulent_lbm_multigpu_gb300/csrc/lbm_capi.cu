@@ -282,105 +282,8 @@ __global__ void k_halo_batch(const __grid_constant__ HaloArgs<N> a) {
     halo_elem<E>(a.h[blockIdx.z]);
 }
 
-// Neumaier-compensated FP64 accumulation.
-struct Acc {
-    double s, c;
-    __device__ __forceinline__ void add(double v) {
-        const double t = s + v;
-        if (fabs(s) >= fabs(v)) c += (s - t) + v;
-        else c += (v - t) + s;
-        s = t;
-    }
-    __device__ __forceinline__ void merge(const Acc &o) {
-        add(o.s);
-        c += o.c;
-    }
-};
-
-constexpr int kRedBlocks = 1024;
-
-template <typename S>
-__global__ void __launch_bounds__(kBlock) k_reduce(LatDesc d, int layout, double *partial) {
-    using R = typename Store<S>::R;
-    __shared__ Acc sh[5][kBlock];
-    Acc a[5];
-    for (int q = 0; q < 5; q++) a[q] = Acc{0.0, 0.0};
-    const S *dd = (const S *)d.dd;
-    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < d.n; c += (int64_t)gridDim.x * blockDim.x) {
-        if (d.flags[c] != kFluid) continue;
-        double r = 0, jx = 0, jy = 0, jz = 0;
-#pragma unroll
-        for (int i = 0; i < 19; i++) {
-            const int slot = layout ? opp(i) : i;
-            const double f = (double)Store<S>::ld(dd + slot * d.pstride + c, weight<R>(slot));
-            r += f;
-            jx += dir_x(i) * f;
-            jy += dir_y(i) * f;
-            jz += dir_z(i) * f;
-        }
-        a[0].add(r);
-        a[1].add(jx);
-        a[2].add(jy);
-        a[3].add(jz);
-        a[4].add(0.5 * (jx * jx + jy * jy + jz * jz));
-    }
-    for (int q = 0; q < 5; q++) sh[q][threadIdx.x] = a[q];
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w)
-            for (int q = 0; q < 5; q++) sh[q][threadIdx.x].merge(sh[q][threadIdx.x + w]);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-        for (int q = 0; q < 5; q++) {
-            partial[(blockIdx.x * 5 + q) * 2] = sh[q][0].s;
-            partial[(blockIdx.x * 5 + q) * 2 + 1] = sh[q][0].c;
-        }
-}
-
-// Velocity difference of two lattices of the same size over the fluid cells
-// of `a`: max |ua - ub|, sum |ua - ub|^2, sum |ub|^2, max |ub|, cell count,
-// with u the momentum of the stored populations in the given slot layouts.
-template <typename SA, typename SB>
-__global__ void __launch_bounds__(kBlock) k_compare(LatDesc a, int la, LatDesc b, int lb, double *partial) {
-    using RA = typename Store<SA>::R;
-    using RB = typename Store<SB>::R;
-    __shared__ double sh[5][kBlock];
-    double mx = 0, se = 0, sr = 0, mr = 0, cnt = 0;
-    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < a.n; c += (int64_t)gridDim.x * blockDim.x) {
-        if (a.flags[c] != kFluid) continue;
-        double ua[3] = {0, 0, 0}, ub[3] = {0, 0, 0};
-#pragma unroll
-        for (int i = 0; i < 19; i++) {
-            const int sa = la ? opp(i) : i, sb = lb ? opp(i) : i;
-            const double fa = (double)Store<SA>::ld((const SA *)a.dd + sa * a.pstride + c, weight<RA>(sa));
-            const double fb = (double)Store<SB>::ld((const SB *)b.dd + sb * b.pstride + c, weight<RB>(sb));
-            ua[0] += dir_x(i) * fa; ua[1] += dir_y(i) * fa; ua[2] += dir_z(i) * fa;
-            ub[0] += dir_x(i) * fb; ub[1] += dir_y(i) * fb; ub[2] += dir_z(i) * fb;
-        }
-        const double d0 = ua[0] - ub[0], d1 = ua[1] - ub[1], d2 = ua[2] - ub[2];
-        const double e2 = d0 * d0 + d1 * d1 + d2 * d2, r2 = ub[0] * ub[0] + ub[1] * ub[1] + ub[2] * ub[2];
-        mx = fmax(mx, sqrt(e2));
-        mr = fmax(mr, sqrt(r2));
-        se += e2;
-        sr += r2;
-        cnt += 1;
-    }
-    sh[0][threadIdx.x] = mx; sh[1][threadIdx.x] = se; sh[2][threadIdx.x] = sr; sh[3][threadIdx.x] = mr;
-    sh[4][threadIdx.x] = cnt;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) {
-            sh[0][threadIdx.x] = fmax(sh[0][threadIdx.x], sh[0][threadIdx.x + w]);
-            sh[1][threadIdx.x] += sh[1][threadIdx.x + w];
-            sh[2][threadIdx.x] += sh[2][threadIdx.x + w];
-            sh[3][threadIdx.x] = fmax(sh[3][threadIdx.x], sh[3][threadIdx.x + w]);
-            sh[4][threadIdx.x] += sh[4][threadIdx.x + w];
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x < 5) partial[blockIdx.x * 5 + threadIdx.x] = sh[threadIdx.x][0];
-}
+// Blocks of a grid-stride pass over a lattice.
+constexpr int kStatBlocks = 1024;
 
 // Classes of the stored 16-bit deviations (fluid cells, all 19 slots):
 // counts of all, zero, subnormal (nonzero below the format's smallest
@@ -428,30 +331,6 @@ __global__ void __launch_bounds__(kBlock) k_dev_stats(LatDesc d, unsigned long l
     }
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_down_sync(0xffffffffu, mx, o));
     if ((threadIdx.x & 31) == 0) atomicMax(maxbits, __float_as_uint(mx));  // non-negative floats order as integers
-}
-
-__global__ void k_compare_final(const double *partial, int nblocks, double *out) {
-    if (threadIdx.x != 0) return;
-    double r[5] = {0, 0, 0, 0, 0};
-    for (int b = 0; b < nblocks; b++) {
-        r[0] = fmax(r[0], partial[b * 5 + 0]);
-        r[1] += partial[b * 5 + 1];
-        r[2] += partial[b * 5 + 2];
-        r[3] = fmax(r[3], partial[b * 5 + 3]);
-        r[4] += partial[b * 5 + 4];
-    }
-    for (int q = 0; q < 5; q++) out[q] = r[q];
-}
-
-__global__ void k_reduce_final(const double *partial, int nblocks, double *out) {
-    if (threadIdx.x >= 5) return;
-    const int q = threadIdx.x;
-    Acc a{0.0, 0.0};
-    for (int b = 0; b < nblocks; b++) {
-        a.add(partial[(b * 5 + q) * 2]);
-        a.c += partial[(b * 5 + q) * 2 + 1];
-    }
-    out[q] = a.s + a.c;
 }
 
 // ------------------------------------------------------------- dispatchers
@@ -509,7 +388,7 @@ static int launch_chunk(int storage, bool pair, int parity, bool les, const Doma
 }
 
 // Streaming multiprocessors of the current device (cached per device).
-static int sm_count() {
+int sm_count() {
     static int cache[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
@@ -1015,65 +894,6 @@ int lbm_cu_halo(lbm_lattice *src, const int so[3], lbm_lattice *dst, const int d
     }
 }
 
-int lbm_cu_reduce_conserved(lbm_lattice *l, int layout, double out[5], void *stream) {
-    if (!l || !out) return fail("NULL argument");
-    const size_t need = (size_t)kRedBlocks * 10 * sizeof(double) + 8 * sizeof(double);
-    if (ensure_stage(l, need)) return -1;
-    double *partial = (double *)l->stage;
-    double *res = partial + (size_t)kRedBlocks * 10;
-    const int blocks = std::min<int64_t>(kRedBlocks, std::max<int64_t>(1, grid_for(l->n)));
-    cudaStream_t st = S(stream);
-    switch (l->storage) {
-        case kF32: k_reduce<float><<<blocks, kBlock, 0, st>>>(l->h, layout & 1, partial); break;
-        case kF64: k_reduce<double><<<blocks, kBlock, 0, st>>>(l->h, layout & 1, partial); break;
-        case kF16: k_reduce<__half><<<blocks, kBlock, 0, st>>>(l->h, layout & 1, partial); break;
-        case kBF16: k_reduce<__nv_bfloat16><<<blocks, kBlock, 0, st>>>(l->h, layout & 1, partial); break;
-        case kC16: k_reduce<c16_t><<<blocks, kBlock, 0, st>>>(l->h, layout & 1, partial); break;
-    }
-    CU(cudaGetLastError());
-    k_reduce_final<<<1, 32, 0, st>>>(partial, blocks, res);
-    CU(cudaGetLastError());
-    CU(cudaMemcpyAsync(out, res, 5 * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CU(cudaStreamSynchronize(st));
-    return 0;
-}
-
-int lbm_cu_compare_velocity(lbm_lattice *a, int layout_a, lbm_lattice *b, int layout_b, double out[5],
-                            void *stream) {
-    if (!a || !b || !out) return fail("NULL argument");
-    if (a->nx != b->nx || a->ny != b->ny || a->nz != b->nz) return fail("lattices differ in size");
-    const size_t need = (size_t)kRedBlocks * 5 * sizeof(double) + 8 * sizeof(double);
-    if (ensure_stage(a, need)) return -1;
-    double *partial = (double *)a->stage;
-    double *res = partial + (size_t)kRedBlocks * 5;
-    const int blocks = std::min<int64_t>(kRedBlocks, std::max<int64_t>(1, grid_for(a->n)));
-    cudaStream_t st = S(stream);
-#define CMP(SA_, SB_) k_compare<SA_, SB_><<<blocks, kBlock, 0, st>>>(a->h, layout_a & 1, b->h, layout_b & 1, partial)
-#define CMPB(SA_)                                   \
-    switch (b->storage) {                           \
-        case kF32: CMP(SA_, float); break;          \
-        case kF64: CMP(SA_, double); break;         \
-        case kF16: CMP(SA_, __half); break;         \
-        case kBF16: CMP(SA_, __nv_bfloat16); break; \
-        case kC16: CMP(SA_, c16_t); break;          \
-    }
-    switch (a->storage) {
-        case kF32: CMPB(float); break;
-        case kF64: CMPB(double); break;
-        case kF16: CMPB(__half); break;
-        case kBF16: CMPB(__nv_bfloat16); break;
-        case kC16: CMPB(c16_t); break;
-    }
-#undef CMPB
-#undef CMP
-    CU(cudaGetLastError());
-    k_compare_final<<<1, 32, 0, st>>>(partial, blocks, res);
-    CU(cudaGetLastError());
-    CU(cudaMemcpyAsync(out, res, 5 * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CU(cudaStreamSynchronize(st));
-    return 0;
-}
-
 int lbm_cu_deviation_stats(lbm_lattice *l, double out[5], void *stream) {
     if (!l || !out) return fail("NULL argument");
     if (l->storage != kF16 && l->storage != kBF16 && l->storage != kC16)
@@ -1083,7 +903,7 @@ int lbm_cu_deviation_stats(lbm_lattice *l, double out[5], void *stream) {
     unsigned int *mx = (unsigned int *)(cnt + 4);
     cudaStream_t st = S(stream);
     CU(cudaMemsetAsync(l->stage, 0, 64, st));
-    const int blocks = std::min<int64_t>(kRedBlocks, std::max<int64_t>(1, grid_for(l->n)));
+    const int blocks = std::min<int64_t>(kStatBlocks, std::max<int64_t>(1, grid_for(l->n)));
     switch (l->storage) {
         case kF16: k_dev_stats<__half><<<blocks, kBlock, 0, st>>>(l->h, cnt, mx); break;
         case kBF16: k_dev_stats<__nv_bfloat16><<<blocks, kBlock, 0, st>>>(l->h, cnt, mx); break;
@@ -1103,88 +923,6 @@ int lbm_cu_deviation_stats(lbm_lattice *l, double out[5], void *stream) {
 }
 
 }  // extern "C"
-
-// ------------------------------------------ reduction without allocation
-// Some callers must not allocate device memory: a serving loop that has
-// handed every free byte of HBM to resident fields under a budget, a monitor
-// thread that checks conservation while other streams run and cannot take
-// the device-wide synchronisation cudaMalloc/cudaFree may imply, or a host
-// framework whose own allocator owns the device.  For them the partial sums
-// of the conservation reduction live in this fixed array instead of the
-// lattice's staging buffer: one partial (sum and compensation of 5
-// quantities) per block of 256 threads x 32 cells, at most kStaticPartials
-// blocks, so lattices of up to kStaticPartials * kStaticCellsPerBlock cells.
-// The array exists once per GPU that loads this library and stays allocated
-// until the process exits.  Every call reuses it: each call writes every
-// partial it later reads, so nothing has to be cleared, but two calls whose
-// work overlaps on the GPU (different streams, no ordering) race on it.
-constexpr int kStaticPartials = 16384;
-constexpr int64_t kStaticCellsPerBlock = (int64_t)kBlock * 32;
-static __device__ __align__(256) double g_reduce_scratch[kStaticPartials * 10 + 8];
-
-// Final stage over up to kStaticPartials partials: warp q sums quantity q,
-// each lane a strided share with its own compensated sum, then the lanes'
-// sums are merged by shuffles (one block of 5 warps; a single thread per
-// quantity would walk all 16384 partials one after another).
-__global__ void __launch_bounds__(160) k_reduce_final_warps(const double *partial, int nblocks, double *out) {
-    const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    Acc a{0.0, 0.0};
-    for (int b = lane; b < nblocks; b += 32) {
-        a.add(partial[(b * 5 + q) * 2]);
-        a.c += partial[(b * 5 + q) * 2 + 1];
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        const Acc other{__shfl_down_sync(0xffffffffu, a.s, o), __shfl_down_sync(0xffffffffu, a.c, o)};
-        if (lane + o < 32) a.merge(other);
-    }
-    if (lane == 0) out[q] = a.s + a.c;
-}
-
-namespace {
-// Device address of g_reduce_scratch, looked up once per device with that
-// device current (the host-side symbol is not a device address).
-int static_scratch(double **out) {
-    static std::mutex mu;
-    static double *addr[128] = {};
-    int dev = 0;
-    CU(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 128) return fail("device ordinal out of range");
-    std::lock_guard<std::mutex> lock(mu);
-    if (!addr[dev]) {
-        void *p = nullptr;
-        CU(cudaGetSymbolAddress(&p, g_reduce_scratch));
-        addr[dev] = (double *)p;
-    }
-    *out = addr[dev];
-    return 0;
-}
-}  // namespace
-
-extern "C" int lbm_cu_reduce_conserved_noalloc(lbm_lattice *l, int layout, double out[5], void *stream) {
-    if (!l || !out) return fail("NULL argument");
-    const int64_t max_cells = (int64_t)kStaticPartials * kStaticCellsPerBlock;
-    if (l->n > max_cells)
-        return fail("lattice has " + std::to_string(l->n) + " cells; the no-allocation reduction handles at most " +
-                    std::to_string(max_cells));
-    double *partial = nullptr;
-    if (static_scratch(&partial)) return -1;
-    double *res = partial + (size_t)kStaticPartials * 10;
-    const int blocks = (int)std::max<int64_t>(1, (l->n + kStaticCellsPerBlock - 1) / kStaticCellsPerBlock);
-    cudaStream_t st = S(stream);
-    switch (l->storage) {
-        case kF32: k_reduce<float><<<blocks, kBlock, 0, st>>>(l->h, layout & 1, partial); break;
-        case kF64: k_reduce<double><<<blocks, kBlock, 0, st>>>(l->h, layout & 1, partial); break;
-        case kF16: k_reduce<__half><<<blocks, kBlock, 0, st>>>(l->h, layout & 1, partial); break;
-        case kBF16: k_reduce<__nv_bfloat16><<<blocks, kBlock, 0, st>>>(l->h, layout & 1, partial); break;
-        case kC16: k_reduce<c16_t><<<blocks, kBlock, 0, st>>>(l->h, layout & 1, partial); break;
-    }
-    CU(cudaGetLastError());
-    k_reduce_final_warps<<<1, 160, 0, st>>>(partial, blocks, res);
-    CU(cudaGetLastError());
-    CU(cudaMemcpyAsync(out, res, 5 * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CU(cudaStreamSynchronize(st));
-    return 0;
-}
 
 // ================================================================== domain
 struct CommGeom {

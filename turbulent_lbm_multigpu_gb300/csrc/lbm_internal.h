@@ -55,6 +55,11 @@ constexpr int kShapeF64Fma = 4;
 // kernels (lbm_f64fma.cu); blocks of kBlock cells.
 int launch_step_f64_fma(int parity, bool les, const DomainArgs &a, int blocks, cudaStream_t st);
 
+// Streaming multiprocessors of the current device (cached per device).
+int sm_count();
+// Grow a lattice's staging buffer to at least `bytes`.
+int ensure_stage(lbm_lattice *l, size_t bytes);
+
 // One step over `ntab` lattices of one storage type, kParamLattices
 // descriptors per launch.
 int launch_step(int storage, int shape, int parity, bool les, const LatDesc *htab, int ntab, int sv, int sr,
