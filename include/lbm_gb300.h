@@ -132,11 +132,13 @@ int lbm_cu_step(lbm_lattice *lat, int parity, void *stream);
  * src/CLbmSolver.hpp:279-312, tunes its OpenCL launch instead). */
 int lbm_cu_set_kernel_shape(lbm_lattice *lat, int cells_per_thread);
 
-/* Double lattices only: enable != 0 runs the step with kernels whose FP64
- * products may fuse into the following sum (one rounding instead of two);
- * 0 (default) keeps the bit-exact reference arithmetic.  A contracted step
- * differs from the reference's by a relative 1e-15 (bound: 1e-12 per step),
- * and runs faster because the double kernels are bound by the FP64 pipe.
+/* Double lattices only: enable != 0 runs the step with kernels that leave out
+ * roundings of the reference arithmetic: sums are exact and products are cut
+ * at 2^-61 in integers (cells of ordinary flows), or fuse into the following
+ * sum in double arithmetic (others).  0 (default) keeps the bit-exact
+ * reference arithmetic.  A contracted step differs from the reference's by a
+ * relative 1e-15 (bound: 1e-12 per step), is closer to the model than it,
+ * and runs faster.
  * One cell per thread; overrides the kernel shape.  No reference counterpart
  * (the reference builds its double kernels with the OpenCL compiler's
  * defaults, src/CLbmSolver.hpp:319-373). */

@@ -206,7 +206,7 @@ class Lattice:
         check(lib().lbm_cu_set_kernel_shape(self.h, cells_per_thread))
 
     def set_fp64_contraction(self, enable: bool):
-        """Double storage: fused multiply-adds in the step (1e-15 per step off the reference arithmetic)."""
+        """Double storage: steps without the reference's intermediate roundings (1e-15 per step off its arithmetic)."""
         check(lib().lbm_cu_set_fp64_contraction(self.h, int(enable)))
 
     def _shape(self, field, size):

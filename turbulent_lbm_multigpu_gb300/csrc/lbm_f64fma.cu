@@ -1,14 +1,15 @@
-// lbm_f64fma.cu -- the one-cell step kernels for double populations with
-// fused multiply-adds.
+// lbm_f64fma.cu -- the one-cell step kernels for double populations without
+// the reference's intermediate roundings.
 //
-// This translation unit is compiled with -fmad=true (every other one with
-// -fmad=false), so the compiler may contract each product that feeds a sum
-// into one FP64 fused multiply-add.  The arithmetic is otherwise the same
-// expressions in the same order as the bit-exact kernels; every contraction
-// rounds once instead of twice, so a step differs from the reference
-// arithmetic by a few units in the last place (a relative 1e-15, well inside
-// the 1e-12 per-step bound for double), while the FP64 pipe -- which bounds
-// the double kernels on GB300, not HBM -- issues fewer operations.
+// Cells of ordinary flows are collided in 62-bit integers (fq_collide,
+// lbm_fix64.cuh): exact sums, products cut at 2^-61, one rounding per
+// population at the end.  Other cells run the double expressions, which this
+// translation unit alone compiles with -fmad=true, so that the compiler may
+// contract each product that feeds a sum into one FP64 fused multiply-add.
+// Either way a step differs from the reference arithmetic by a few units in
+// the last place (a relative 1e-15, well inside the 1e-12 per-step bound for
+// double); against 128-bit arithmetic the integer form is off by 4e-17 RMS
+// where fused double arithmetic is off by 2.3e-16.
 //
 // The kernels are instantiated for a storage tag type of their own (F64Fma:
 // one double), so that their template instances can never be confused with
