@@ -34,28 +34,20 @@ template <typename S, bool PAIR>
 int launch_tick_t(bool les, const BatchArgs &a, int blocks, int j, int uni, cudaStream_t st) {
     if (blocks <= 0) return 0;
     if constexpr (PAIR) {
-        if (les) k_step2<S, true><<<blocks, kBlock, 0, st>>>(a, j);
-        else k_step2<S, false><<<blocks, kBlock, 0, st>>>(a, j);
+        return les ? launch_dep(k_step2<S, true>, blocks, kBlock, 0, st, a, j)
+                   : launch_dep(k_step2<S, false>, blocks, kBlock, 0, st, a, j);
     } else if constexpr (sizeof(S) >= 4) {
         // float and double chunks whose cavities are all at the same kind of
         // step run that kind's kernel alone (its own launch bounds)
-        if (uni == 1) {
-            if (les) k_step<S, true, 1><<<blocks, kBlock, 0, st>>>(a, j);
-            else k_step<S, false, 1><<<blocks, kBlock, 0, st>>>(a, j);
-        } else if (uni == 2) {
-            if (les) k_step<S, true, 2><<<blocks, kBlock, 0, st>>>(a, j);
-            else k_step<S, false, 2><<<blocks, kBlock, 0, st>>>(a, j);
-        } else {
-            if (les) k_step<S, true><<<blocks, kBlock, 0, st>>>(a, j);
-            else k_step<S, false><<<blocks, kBlock, 0, st>>>(a, j);
-        }
-    } else {
-        (void)uni;
-        if (les) k_step<S, true><<<blocks, kBlock, 0, st>>>(a, j);
-        else k_step<S, false><<<blocks, kBlock, 0, st>>>(a, j);
+        if (uni == 1)
+            return les ? launch_dep(k_step<S, true, 1>, blocks, kBlock, 0, st, a, j)
+                       : launch_dep(k_step<S, false, 1>, blocks, kBlock, 0, st, a, j);
+        if (uni == 2)
+            return les ? launch_dep(k_step<S, true, 2>, blocks, kBlock, 0, st, a, j)
+                       : launch_dep(k_step<S, false, 2>, blocks, kBlock, 0, st, a, j);
     }
-    CU(cudaGetLastError());
-    return 0;
+    return les ? launch_dep(k_step<S, true>, blocks, kBlock, 0, st, a, j)
+               : launch_dep(k_step<S, false>, blocks, kBlock, 0, st, a, j);
 }
 
 int launch_tick(int storage, bool pair, bool les, const BatchArgs &a, int blocks, int j, int uni, cudaStream_t st) {
@@ -386,8 +378,10 @@ extern "C" {
 // ---------------------------------------------------------------- one lattice
 int lbm_cu_run(lbm_lattice *lat, int64_t first_step, int64_t steps, void *stream) {
     if (!lat) return fail("NULL lattice");
+    // every step writes u and rho of the same cells, so only the last step's
+    // can be read after the run (16 of a float cell's 168 bytes)
     for (int64_t t = 0; t < steps; t++)
-        if (lbm_cu_step(lat, (int)((first_step + t) & 1), stream)) return -1;
+        if (step_lattice(lat, (int)((first_step + t) & 1), t + 1 == steps, S(stream))) return -1;
     return 0;
 }
 

@@ -279,6 +279,7 @@ static_assert(sizeof(HaloArgs<kHaloParam>) <= 32764, "halo descriptors exceed th
 
 template <typename E, int N>
 __global__ void k_halo_batch(const __grid_constant__ HaloArgs<N> a) {
+    follow_previous_grid();
     halo_elem<E>(a.h[blockIdx.z]);
 }
 
@@ -337,17 +338,10 @@ __global__ void __launch_bounds__(kBlock) k_dev_stats(LatDesc d, unsigned long l
 template <typename S, bool PAIR>
 int launch_step_t(int parity, bool les, const DomainArgs &a, int blocks, cudaStream_t st) {
     if (blocks <= 0) return 0;
-#define STEP(K_, L_) K_<S, L_><<<blocks, kBlock, 0, st>>>(a)
-    if constexpr (PAIR) {
-        if (parity) { if (les) STEP(k_alpha2, true); else STEP(k_alpha2, false); }
-        else { if (les) STEP(k_beta2, true); else STEP(k_beta2, false); }
-    } else {
-        if (parity) { if (les) STEP(k_alpha, true); else STEP(k_alpha, false); }
-        else { if (les) STEP(k_beta, true); else STEP(k_beta, false); }
-    }
+#define STEP(K_) (les ? launch_dep(K_<S, true>, blocks, kBlock, 0, st, a) : launch_dep(K_<S, false>, blocks, kBlock, 0, st, a))
+    if constexpr (PAIR) return parity ? STEP(k_alpha2) : STEP(k_beta2);
+    else return parity ? STEP(k_alpha) : STEP(k_beta);
 #undef STEP
-    CU(cudaGetLastError());
-    return 0;
 }
 
 // The two-cell kernels apply to the float arithmetic types when every
@@ -414,9 +408,7 @@ static int launch_staged_w(const StepArgs<N> &a, int tiles, cudaStream_t st) {
         attr[dev] = true;
     }
     const int grid = std::min(tiles, sm_count() * kStageBlocksPerSM);
-    k_step_staged<S, LES, BETA, ONE, N, ADDR><<<grid, kStageThreads, Tile<S>::SMEM, st>>>(a, tiles);
-    CU(cudaGetLastError());
-    return 0;
+    return launch_dep(k_step_staged<S, LES, BETA, ONE, N, ADDR>, grid, kStageThreads, Tile<S>::SMEM, st, a, tiles);
 }
 
 // Beta steps whose lattices all span fewer than 2^32 population elements
@@ -547,6 +539,13 @@ int launch_step(int storage, int shape, int parity, bool les, const LatDesc *hta
     return 0;
 }
 
+int step_lattice(const lbm_lattice *l, int parity, bool store, cudaStream_t st) {
+    const LatDesc &h = l->h;
+    const int shape = l->fma64 && l->storage == kF64 ? kShapeF64Fma : effective_shape(l->storage, l->shape, &h, 1);
+    return launch_step(l->storage, shape, parity & 1, uses_les(h), &h, 1, store ? l->store_v : 0,
+                       store ? l->store_rho : 0, st);
+}
+
 Box make_box(const lbm_lattice *l, const int o[3], const int s[3]) {
     Box b;
     b.lat_nx = l->nx;
@@ -584,9 +583,7 @@ static int launch_halo_param(const HaloDesc *hd, int n, int64_t max_cells, int m
     HaloArgs<N> a;
     memset(&a, 0, sizeof(a));
     memcpy(a.h, hd, (size_t)n * sizeof(HaloDesc));
-    k_halo_batch<E, N><<<halo_grid(max_cells, max_planes, n), kBlock, 0, st>>>(a);
-    CU(cudaGetLastError());
-    return 0;
+    return launch_dep(k_halo_batch<E, N>, halo_grid(max_cells, max_planes, n), kBlock, 0, st, a);
 }
 
 template <typename E>
@@ -757,10 +754,7 @@ int lbm_cu_perturb(lbm_lattice *l, const int o[3], const int ph[3], uint64_t see
 
 int lbm_cu_step(lbm_lattice *l, int parity, void *stream) {
     if (!l) return fail("NULL lattice");
-    const LatDesc &h = l->h;
-    const int shape = l->fma64 && l->storage == kF64 ? kShapeF64Fma : effective_shape(l->storage, l->shape, &h, 1);
-    return launch_step(l->storage, shape, parity & 1, uses_les(h), &h, 1,
-                       l->store_v, l->store_rho, S(stream));
+    return step_lattice(l, parity, true, S(stream));
 }
 
 static int box_io(lbm_lattice *l, int field, const int o[3], const int s[3], void *host, const int norm[3],

@@ -24,6 +24,28 @@ int fail(const std::string &m);
 
 inline cudaStream_t S(void *s) { return (cudaStream_t)s; }
 
+// Launch of a kernel that begins with follow_previous_grid(): its blocks may
+// be set up while the grid before it on the stream drains.  Measured on runs
+// launched step by step (us per step, plain -> this): float 24^3 5.17 -> 3.48,
+// 64^3 9.20 -> 6.90, 128^3 54.9 -> 53.1, 256^3 398.6 -> 396.1; half 24^3
+// 6.71 -> 4.94, 128^3 31.9 -> 30.5: about 2 us a launch.  Replayed from a
+// captured graph the same kernels gain nothing (24^3 4.14 -> 4.11).
+template <typename... P, typename... A>
+inline int launch_dep(void (*kernel)(P...), dim3 grid, int threads, size_t shared, cudaStream_t st, const A &...args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = shared;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    CU(cudaLaunchKernelEx(&cfg, kernel, args...));
+    return 0;
+}
+
 constexpr int kBlock = 256;
 
 inline size_t storage_bytes(int st) { return st == kF64 ? 8 : st == kF32 ? 4 : 2; }
@@ -64,6 +86,9 @@ int ensure_stage(lbm_lattice *l, size_t bytes);
 // descriptors per launch.
 int launch_step(int storage, int shape, int parity, bool les, const LatDesc *htab, int ntab, int sv, int sr,
                 cudaStream_t st);
+// One step of a lattice in its own kernel shape; store: write u and rho, if
+// the lattice keeps them.
+int step_lattice(const lbm_lattice *l, int parity, bool store, cudaStream_t st);
 // Cells per staged tile of a storage type (0: not staged).
 int staged_cells(int storage);
 // One step of up to kBatchLattices lattices, all at an alpha step or all at
