@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "lbm_internal.h"
+#include "lbm_startup.cuh"
 
 using namespace lbm;
 using namespace lbm_rt;
@@ -102,20 +103,17 @@ lbm_params cavity_params(const lbm_cavity &c) {
     return p;
 }
 
-// A lid-driven cavity at step 0: walls on all faces, the lid plane of
-// CController::setGeometry (src/CController.hpp:531-546), optional seeded
-// start-up.
+// A lid-driven cavity at step 0, asynchronously (k_cavity).
 int cavity_reset(lbm_lattice *l, const lbm_cavity &c, cudaStream_t st) {
-    const int bc[6] = {LBM_FLAG_OBSTACLE, LBM_FLAG_OBSTACLE, LBM_FLAG_OBSTACLE,
-                       LBM_FLAG_OBSTACLE, LBM_FLAG_OBSTACLE, LBM_FLAG_OBSTACLE};
-    if (lbm_cu_init(l, bc, st)) return -1;
-    const int o[3] = {1, c.ny - 2, 1}, sz[3] = {c.nx - 2, 1, c.nz - 2};
-    std::vector<int32_t> lid((size_t)sz[0] * sz[2], LBM_FLAG_VELOCITY_INJECTION);
-    if (lbm_cu_write(l, LBM_FIELD_FLAGS, o, sz, lid.data(), nullptr, st)) return -1;
-    if (c.amp != 0.0) {
-        const int zero[3] = {0, 0, 0}, phys[3] = {c.nx, c.ny, c.nz};
-        if (lbm_cu_perturb(l, zero, phys, c.seed, c.amp, st)) return -1;
+    const int g = grid_for(l->n);
+    switch (l->storage) {
+        case kF32: k_cavity<float><<<g, kBlock, 0, st>>>(l->h, c.seed, c.amp, l->store_v); break;
+        case kF64: k_cavity<double><<<g, kBlock, 0, st>>>(l->h, c.seed, c.amp, l->store_v); break;
+        case kF16: k_cavity<__half><<<g, kBlock, 0, st>>>(l->h, c.seed, c.amp, l->store_v); break;
+        case kBF16: k_cavity<__nv_bfloat16><<<g, kBlock, 0, st>>>(l->h, c.seed, c.amp, l->store_v); break;
+        case kC16: k_cavity<c16_t><<<g, kBlock, 0, st>>>(l->h, c.seed, c.amp, l->store_v); break;
     }
+    CU(cudaGetLastError());
     return 0;
 }
 

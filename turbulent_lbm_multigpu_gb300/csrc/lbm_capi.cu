@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "lbm_internal.h"
+#include "lbm_startup.cuh"
 
 using namespace lbm;
 using namespace lbm_rt;
@@ -92,7 +93,8 @@ __global__ void k_init(LatDesc d, int b0, int b1, int b2, int b3, int b4, int b5
     using R = typename Store<S>::R;
     const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= d.n) return;
-    const int64_t x = c % d.nx, y = (c / d.nx) % d.ny, z = c / ((int64_t)d.nx * d.ny);
+    const uint32_t cc = (uint32_t)c, row = cc / (uint32_t)d.nx;  // n < 2^31
+    const int x = (int)(cc - row * (uint32_t)d.nx), y = (int)(row % (uint32_t)d.ny), z = (int)(row / (uint32_t)d.ny);
     int fl = kFluid;  // x faces win over y faces, y over z (lbm_init.cl:53-68)
     if (x == 0) fl = b0;
     else if (x == d.nx - 1) fl = b1;
@@ -114,37 +116,18 @@ __global__ void k_init(LatDesc d, int b0, int b1, int b2, int b3, int b4, int b5
     if (store_rho) ((R *)d.rho)[c] = (R)1.0f;
 }
 
-// Philox4x32-10 (Salmon et al., SC'11), same as the oracle's.
-__device__ void philox(uint32_t c[4], uint32_t k0, uint32_t k1) {
-    for (int r = 0; r < 10; r++) {
-        const uint64_t p0 = (uint64_t)0xD2511F53u * c[0];
-        const uint64_t p1 = (uint64_t)0xCD9E8D57u * c[2];
-        const uint32_t n0 = (uint32_t)(p1 >> 32) ^ c[1] ^ k0;
-        const uint32_t n1 = (uint32_t)p1;
-        const uint32_t n2 = (uint32_t)(p0 >> 32) ^ c[3] ^ k1;
-        const uint32_t n3 = (uint32_t)p0;
-        c[0] = n0; c[1] = n1; c[2] = n2; c[3] = n3;
-        k0 += 0x9E3779B9u;
-        k1 += 0xBB67AE85u;
-    }
-}
-
 template <typename S>
 __global__ void k_perturb(LatDesc d, int ox, int oy, int oz, int gx, int gy, int gz, uint64_t seed, double amp,
                           int store_v, int store_rho) {
     using R = typename Store<S>::R;
     const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= d.n) return;
-    const int64_t px = ox + c % d.nx, py = oy + (c / d.nx) % d.ny, pz = oz + c / ((int64_t)d.nx * d.ny);
+    const uint32_t cc = (uint32_t)c, row = cc / (uint32_t)d.nx;  // n < 2^31
+    const int64_t px = ox + (int64_t)(cc - row * (uint32_t)d.nx), py = oy + (int64_t)(row % (uint32_t)d.ny),
+                  pz = oz + (int64_t)(row / (uint32_t)d.ny);
     if (px <= 0 || py <= 0 || pz <= 0 || px >= gx - 1 || py >= gy - 1 || pz >= gz - 1) return;
-    const uint64_t idx = (uint64_t)((pz * gy + py) * gx + px);
-    uint32_t r[4] = {(uint32_t)idx, (uint32_t)(idx >> 32), 0u, 0u};
-    philox(r, (uint32_t)seed, (uint32_t)(seed >> 32));
     R u[3];
-    for (int a = 0; a < 3; a++) {
-        const double unit = (double)(r[a] >> 8) * (1.0 / 16777216.0);
-        u[a] = (R)((unit * 2.0 - 1.0) * amp);
-    }
+    startup_velocity<R>((uint64_t)((pz * gy + py) * gx + px), seed, amp, u);
     const R v2 = (u[0] * u[0] + u[1] * u[1]) + u[2] * u[2];
     const R dp = (R)1.0f - K<R>::k15 * v2;
     R eq[19];
