@@ -338,8 +338,9 @@ int lbm_cu_run(lbm_lattice *lat, int64_t first_step, int64_t steps, void *stream
 
 /* An ensemble of cavities of different sizes, parameters, storage types and
  * step counts, all resident, advanced together: one launch per storage type
- * and step covers every unfinished cavity, pairs of steps replay a captured
- * CUDA graph, every cavity stops at its own step count.  Each cavity's
+ * and step covers every unfinished cavity, every cavity stops at its own
+ * step count (pairs of steps of small ensembles replay a captured CUDA graph
+ * when use_graph != 0).  Each cavity's
  * fields are the same as when it runs alone (lbm_cu_batch_lattice gives
  * its lattice for readback; velocity is written on its last step when
  * store_velocity is set). */
@@ -365,7 +366,9 @@ lbm_lattice *lbm_cu_batch_lattice(lbm_batch *b, int index);
  * HBM budget (and fewer than max_active run), advances every running solve
  * by up to max_steps steps in shared launches (stopping when the first one
  * completes), and retires completed solves, whose fields stay resident
- * until released.  A solve's result does not depend on what else runs. */
+ * until released.  A released solve's device memory is kept for later ones,
+ * at most an eighth of the budget (all of it within the budget), and freed
+ * with the server.  A solve's result does not depend on what else runs. */
 int lbm_cu_server_create(double hbm_budget_bytes, int max_active, int store_velocity, lbm_server **out);
 int lbm_cu_server_destroy(lbm_server *s);
 /* As lbm_cu_batch_set_kernel_shape; a server starts with shape 3. */

@@ -32,41 +32,41 @@ using namespace lbm_rt;
 namespace lbm_rt {
 
 template <typename S, bool PAIR>
-int launch_tick_t(bool les, const BatchArgs &a, int blocks, int j, int uni, cudaStream_t st) {
+int launch_tick_t(bool les, const BatchArgs &a, int blocks, int j, int uni, Dep dep, cudaStream_t st) {
     if (blocks <= 0) return 0;
     if constexpr (PAIR) {
-        return les ? launch_dep(k_step2<S, true>, blocks, kBlock, 0, st, a, j)
-                   : launch_dep(k_step2<S, false>, blocks, kBlock, 0, st, a, j);
+        return les ? launch_dep(dep, k_step2<S, true>, blocks, kBlock, 0, st, a, j)
+                   : launch_dep(dep, k_step2<S, false>, blocks, kBlock, 0, st, a, j);
     } else if constexpr (sizeof(S) >= 4) {
         // float and double chunks whose cavities are all at the same kind of
         // step run that kind's kernel alone (its own launch bounds)
         if (uni == 1)
-            return les ? launch_dep(k_step<S, true, 1>, blocks, kBlock, 0, st, a, j)
-                       : launch_dep(k_step<S, false, 1>, blocks, kBlock, 0, st, a, j);
+            return les ? launch_dep(dep, k_step<S, true, 1>, blocks, kBlock, 0, st, a, j)
+                       : launch_dep(dep, k_step<S, false, 1>, blocks, kBlock, 0, st, a, j);
         if (uni == 2)
-            return les ? launch_dep(k_step<S, true, 2>, blocks, kBlock, 0, st, a, j)
-                       : launch_dep(k_step<S, false, 2>, blocks, kBlock, 0, st, a, j);
+            return les ? launch_dep(dep, k_step<S, true, 2>, blocks, kBlock, 0, st, a, j)
+                       : launch_dep(dep, k_step<S, false, 2>, blocks, kBlock, 0, st, a, j);
     }
-    return les ? launch_dep(k_step<S, true>, blocks, kBlock, 0, st, a, j)
-               : launch_dep(k_step<S, false>, blocks, kBlock, 0, st, a, j);
+    return les ? launch_dep(dep, k_step<S, true>, blocks, kBlock, 0, st, a, j)
+               : launch_dep(dep, k_step<S, false>, blocks, kBlock, 0, st, a, j);
 }
 
-int launch_tick(int storage, bool pair, bool les, const BatchArgs &a, int blocks, int j, int uni, cudaStream_t st) {
+int launch_tick(int storage, bool pair, bool les, const BatchArgs &a, int blocks, int j, int uni, Dep dep, cudaStream_t st) {
     if (pair) {
         switch (storage) {
-            case kF32: return launch_tick_t<float, true>(les, a, blocks, j, uni, st);
-            case kF16: return launch_tick_t<__half, true>(les, a, blocks, j, uni, st);
-            case kBF16: return launch_tick_t<__nv_bfloat16, true>(les, a, blocks, j, uni, st);
-            case kC16: return launch_tick_t<c16_t, true>(les, a, blocks, j, uni, st);
+            case kF32: return launch_tick_t<float, true>(les, a, blocks, j, uni, dep, st);
+            case kF16: return launch_tick_t<__half, true>(les, a, blocks, j, uni, dep, st);
+            case kBF16: return launch_tick_t<__nv_bfloat16, true>(les, a, blocks, j, uni, dep, st);
+            case kC16: return launch_tick_t<c16_t, true>(les, a, blocks, j, uni, dep, st);
         }
         return fail("the two-cell kernels need a float arithmetic type");
     }
     switch (storage) {
-        case kF32: return launch_tick_t<float, false>(les, a, blocks, j, uni, st);
-        case kF64: return launch_tick_t<double, false>(les, a, blocks, j, uni, st);
-        case kF16: return launch_tick_t<__half, false>(les, a, blocks, j, uni, st);
-        case kBF16: return launch_tick_t<__nv_bfloat16, false>(les, a, blocks, j, uni, st);
-        case kC16: return launch_tick_t<c16_t, false>(les, a, blocks, j, uni, st);
+        case kF32: return launch_tick_t<float, false>(les, a, blocks, j, uni, dep, st);
+        case kF64: return launch_tick_t<double, false>(les, a, blocks, j, uni, dep, st);
+        case kF16: return launch_tick_t<__half, false>(les, a, blocks, j, uni, dep, st);
+        case kBF16: return launch_tick_t<__nv_bfloat16, false>(les, a, blocks, j, uni, dep, st);
+        case kC16: return launch_tick_t<c16_t, false>(les, a, blocks, j, uni, dep, st);
     }
     return fail("unknown storage type");
 }
@@ -117,10 +117,22 @@ int cavity_reset(lbm_lattice *l, const lbm_cavity &c, cudaStream_t st) {
     return 0;
 }
 
+// Where a tick replays its pairs of steps from a graph.  Launched one by one
+// with programmatic dependent launch the steps follow one another faster on
+// the GPU, but a launch with its 31 KB of descriptors takes the host about
+// 5 us: ensembles whose steps are shorter than that are replayed.  Measured
+// (half float, half half, us per step, graph / launches): 4 cavities of 24^3
+// 9.5 / 11.4, 4 of 32^3 13.9 / 12.5, 16 of 40^3 27.9 / 25.2, 2 of 96^3 41.7 /
+// 39.4.  Capturing a pair costs as much as ten pairs' launches.
+constexpr int64_t kGraphSteps = 24;
+constexpr int64_t kGraphCells = 96 * 1024;
+
 struct Ensemble {
     struct Slot {
         lbm_cavity spec{};
         lbm_lattice *lat = nullptr;
+        void *block = nullptr;  // a server's device block under the lattice
+        size_t block_bytes = 0;
         int64_t done = 0;
         bool active = false;
         int64_t id = -1;
@@ -141,7 +153,6 @@ struct Ensemble {
         bool aligned = false;  // staged, and every nx a multiple of 16 bytes: beta steps staged too
         std::vector<int> members;
         std::vector<Chunk> chunks;
-        int32_t *dmap = nullptr;  // lattice index (within its chunk) of every block
     };
     std::vector<Slot> slots;
     std::vector<Group> groups;
@@ -155,7 +166,6 @@ struct Ensemble {
     ~Ensemble() {
         drop_graph();
         if (cap) cudaStreamDestroy(cap);
-        free_groups();
         for (auto &s : slots)
             if (s.lat) lbm_cu_destroy(s.lat);
     }
@@ -163,16 +173,9 @@ struct Ensemble {
         if (graph) cudaGraphExecDestroy(graph);
         graph = nullptr;
     }
-    void free_groups() {
-        for (auto &g : groups)
-            if (g.dmap) cudaFree(g.dmap);
-        groups.clear();
-    }
-
-    // Member groups of the active cavities, one per (storage, shape), and
-    // their block maps.
+    // Member groups of the active cavities, one per (storage, shape).
     int build_groups() {
-        free_groups();
+        groups.clear();
         for (size_t i = 0; i < slots.size(); i++) {
             const Slot &s = slots[i];
             if (!s.active) continue;
@@ -194,14 +197,6 @@ struct Ensemble {
             g->members.push_back((int)i);
         }
         for (auto &g : groups) {
-            const int per = cells_per_block(g.pair);
-            std::vector<int32_t> map;
-            for (size_t k = 0; k < g.members.size(); k++) {
-                const int64_t n = slots[g.members[k]].lat->n;
-                map.insert(map.end(), (size_t)((n + per - 1) / per), (int32_t)(k % kBatchLattices));
-            }
-            CU(cudaMalloc((void **)&g.dmap, map.size() * sizeof(int32_t)));
-            CU(cudaMemcpy(g.dmap, map.data(), map.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
             g.chunks.resize((g.members.size() + kBatchLattices - 1) / kBatchLattices);
             for (auto &c : g.chunks) {
                 c.args.reset(new BatchArgs());
@@ -220,7 +215,6 @@ struct Ensemble {
         std::vector<int> parity;
         for (auto &g : groups) {
             const int per = cells_per_block(g.pair);
-            int64_t map_off = 0;
             for (size_t c = 0; c < g.chunks.size(); c++) {
                 Chunk &ch = g.chunks[c];
                 BatchArgs &a = *ch.args;
@@ -240,6 +234,7 @@ struct Ensemble {
                     first += h.nblocks;
                     if (uses_les(h)) ch.les = true;
                     a.tab[k - k0] = h;
+                    a.first[k - k0] = h.first_block;
                     parity.push_back(h.parity);
                     ch.parities |= 1 << h.parity;
                     if (g.staged) {
@@ -247,12 +242,11 @@ struct Ensemble {
                         h.nblocks = (int)((h.n + tcells - 1) / tcells);
                         tile += h.nblocks;
                         ch.sargs->tab[k - k0] = h;
+                        ch.sargs->first[k - k0] = h.first_block;
                     }
                 }
                 a.ntab = (int)(k1 - k0);
-                a.block_lattice = g.dmap + map_off;
                 ch.blocks = first;
-                map_off += first;
                 if (g.staged) ch.sargs->ntab = a.ntab;
                 ch.tiles = tile;
             }
@@ -262,7 +256,7 @@ struct Ensemble {
         return 0;
     }
 
-    int launch_all(int j, bool store, cudaStream_t st) {
+    int launch_all(int j, bool store, Dep dep, cudaStream_t st) {
         for (auto &g : groups)
             for (auto &ch : g.chunks) {
                 const bool all_alpha = ch.parities == 1 << ((j + 1) & 1);
@@ -271,12 +265,12 @@ struct Ensemble {
                     // every member at the same kind of step: staged tiles
                     ch.sargs->store_v = store ? store_v : 0;
                     ch.sargs->store_rho = 0;
-                    if (launch_staged_batch(g.storage, all_beta, ch.les, *ch.sargs, ch.tiles, st)) return -1;
+                    if (launch_staged_batch(g.storage, all_beta, ch.les, *ch.sargs, ch.tiles, dep, st)) return -1;
                     continue;
                 }
                 ch.args->store_v = store ? store_v : 0;
                 ch.args->store_rho = 0;
-                if (launch_tick(g.storage, g.pair, ch.les, *ch.args, ch.blocks, j, all_alpha ? 1 : all_beta ? 2 : 0, st))
+                if (launch_tick(g.storage, g.pair, ch.les, *ch.args, ch.blocks, j, all_alpha ? 1 : all_beta ? 2 : 0, dep, st))
                     return -1;
             }
         return 0;
@@ -288,10 +282,17 @@ struct Ensemble {
         return n;
     }
 
+    int64_t active_cells() const {
+        int64_t n = 0;
+        for (auto &s : slots)
+            if (s.active) n += s.lat->n;
+        return n;
+    }
+
     // Advance every active cavity by k steps; the last step writes u.
     int tick(int64_t k, bool use_graph, cudaStream_t st) {
         if (k <= 0 || active_count() == 0) return 0;
-        CU(cudaStreamSynchronize(st));
+        // nothing here waits for the GPU: descriptors travel with the launches
         if (dirty) {
             if (build_groups()) return -1;
         } else if (refresh_tables()) {
@@ -299,13 +300,13 @@ struct Ensemble {
         }
         const int64_t plain = k - 1;
         int64_t j = 0;
-        if (use_graph && plain >= 2) {
+        if (use_graph && plain >= kGraphSteps && active_cells() < kGraphCells) {
             if (!graph) {
                 if (!cap) CU(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
                 cudaGraph_t g = nullptr;
                 CU(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
-                int rc = launch_all(0, false, cap);
-                if (!rc) rc = launch_all(1, false, cap);
+                int rc = launch_all(0, false, Dep{false}, cap);
+                if (!rc) rc = launch_all(1, false, Dep{false}, cap);
                 cudaError_t e = cudaStreamEndCapture(cap, &g);
                 if (rc) {
                     if (g) cudaGraphDestroy(g);
@@ -324,8 +325,8 @@ struct Ensemble {
             j = 2 * reps;
         }
         for (; j < plain; j++)
-            if (launch_all((int)(j & 1), false, st)) return -1;
-        if (launch_all((int)((k - 1) & 1), true, st)) return -1;
+            if (launch_all((int)(j & 1), false, Dep{}, st)) return -1;
+        if (launch_all((int)((k - 1) & 1), true, Dep{}, st)) return -1;
         for (auto &s : slots)
             if (s.active) s.done += k;
         return 0;
@@ -359,6 +360,61 @@ struct lbm_server {
     Ensemble e;
     double budget = 0;  // bytes of HBM the resident solves may hold
     double used = 0;
+    // Device blocks, one per resident solve.  A released solve's block is
+    // kept for a later one, at most an eighth of the budget of them and all
+    // of them within it (cudaMalloc and cudaFree of a solve's fields took a
+    // tenth of a burst's time).  The device has finished with a block when it
+    // changes hands (release); the server frees them when it is destroyed.
+    struct Block {
+        void *p;
+        size_t bytes;
+    };
+    std::vector<Block> idle;
+    double held = 0, idle_bytes = 0;  // bytes of all blocks, of the idle ones
+
+    ~lbm_server() {
+        for (auto &sl : e.slots) {
+            if (sl.lat) lbm_cu_destroy(sl.lat);
+            sl.lat = nullptr;
+            if (sl.block) cudaFree(sl.block);
+        }
+        while (!idle.empty()) drop_idle(0);
+    }
+    void drop_idle(size_t i) {
+        cudaFree(idle[i].p);
+        held -= (double)idle[i].bytes;
+        idle_bytes -= (double)idle[i].bytes;
+        idle.erase(idle.begin() + i);
+    }
+    // A block of at least `bytes`: the smallest idle one that is no more than
+    // a quarter larger and fits the budget, else a new one.
+    int take(size_t bytes, Block *out) {
+        size_t best = idle.size();
+        for (size_t i = 0; i < idle.size(); i++)
+            if (idle[i].bytes >= bytes && idle[i].bytes <= bytes + bytes / 4 &&
+                held - idle_bytes + (double)idle[i].bytes <= budget && (best == idle.size() || idle[i].bytes < idle[best].bytes))
+                best = i;
+        if (best < idle.size()) {
+            *out = idle[best];
+            idle_bytes -= (double)idle[best].bytes;
+            idle.erase(idle.begin() + best);
+            return 0;
+        }
+        while (!idle.empty() && held + (double)bytes > budget) drop_idle(0);
+        out->bytes = bytes;
+        while (cudaMalloc(&out->p, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            if (idle.empty()) return fail("cudaMalloc of a solve's fields failed");
+            drop_idle(0);
+        }
+        held += (double)bytes;
+        return 0;
+    }
+    void give(Block b) {
+        idle.push_back(b);
+        idle_bytes += (double)b.bytes;
+        while (idle_bytes > budget / 8) drop_idle(0);
+    }
     int max_active = 0;
     int64_t next_id = 0;
     struct Pending {
@@ -429,6 +485,7 @@ int lbm_cu_batch_reset(lbm_batch *b, void *stream) {
         s.active = s.spec.steps > 0;
     }
     b->e.dirty = true;
+    CU(cudaStreamSynchronize(S(stream)));  // a run may use another stream
     return 0;
 }
 
@@ -551,16 +608,24 @@ static int server_admit(lbm_server *s, cudaStream_t st) {
     while (!s->queue.empty()) {
         const lbm_server::Pending &p = s->queue.front();
         const double need = (double)cavity_bytes(p.spec, s->e.store_v);
-        if (s->used + need > s->budget || s->e.active_count() >= s->max_active) break;
+        const size_t bytes = lattice_block_bytes(p.spec.nx, p.spec.ny, p.spec.nz, p.spec.storage, s->e.store_v);
+        if (s->used + need > s->budget || s->held - s->idle_bytes + (double)bytes > s->budget ||
+            s->e.active_count() >= s->max_active)
+            break;
         Ensemble::Slot slot;
         slot.spec = p.spec;
         slot.id = p.id;
-        if (lbm_cu_create(p.spec.nx, p.spec.ny, p.spec.nz, p.spec.storage, s->e.store_v, 0, &slot.lat)) return -1;
+        lbm_server::Block blk{};
+        if (s->take(bytes, &blk)) return -1;
         const lbm_params prm = cavity_params(p.spec);
-        if (lbm_cu_set_params(slot.lat, &prm) || cavity_reset(slot.lat, p.spec, st)) {
+        if (lattice_in_block(p.spec.nx, p.spec.ny, p.spec.nz, p.spec.storage, s->e.store_v, blk.p, &slot.lat) ||
+            lbm_cu_set_params(slot.lat, &prm) || cavity_reset(slot.lat, p.spec, st)) {
             lbm_cu_destroy(slot.lat);
+            s->give(blk);
             return -1;
         }
+        slot.block = blk.p;
+        slot.block_bytes = blk.bytes;
         slot.active = p.spec.steps > 0;
         if (!slot.active) s->completed.push_back(p.id);  // nothing to run
         if (!s->free_slots.empty()) {
@@ -626,8 +691,11 @@ int lbm_cu_server_release(lbm_server *s, int64_t id) {
         auto &sl = s->e.slots[i];
         if (sl.lat && sl.id == id) {
             if (sl.active) return fail("solve is still running");
+            // the caller's own work on the lattice, whatever its stream, ends before the block changes hands
+            CU(cudaDeviceSynchronize());
             s->used -= (double)cavity_bytes(sl.spec, s->e.store_v);
             lbm_cu_destroy(sl.lat);
+            s->give({sl.block, sl.block_bytes});
             sl = Ensemble::Slot();
             s->free_slots.push_back((int)i);
             return 0;

@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(kBlock) k_dev_stats(LatDesc d, unsigned long l
 template <typename S, bool PAIR>
 int launch_step_t(int parity, bool les, const DomainArgs &a, int blocks, cudaStream_t st) {
     if (blocks <= 0) return 0;
-#define STEP(K_) (les ? launch_dep(K_<S, true>, blocks, kBlock, 0, st, a) : launch_dep(K_<S, false>, blocks, kBlock, 0, st, a))
+#define STEP(K_) (les ? launch_dep(Dep{}, K_<S, true>, blocks, kBlock, 0, st, a) : launch_dep(Dep{}, K_<S, false>, blocks, kBlock, 0, st, a))
     if constexpr (PAIR) return parity ? STEP(k_alpha2) : STEP(k_beta2);
     else return parity ? STEP(k_alpha) : STEP(k_beta);
 #undef STEP
@@ -378,7 +378,7 @@ int sm_count() {
 }
 
 template <typename S, bool LES, bool BETA, bool ONE, int N, int ADDR>
-static int launch_staged_w(const StepArgs<N> &a, int tiles, cudaStream_t st) {
+static int launch_staged_w(const StepArgs<N> &a, int tiles, Dep dep, cudaStream_t st) {
     // the ring exceeds the default 48 KB of dynamic shared memory; the limit
     // is raised once per device
     static bool attr[64] = {};
@@ -391,7 +391,7 @@ static int launch_staged_w(const StepArgs<N> &a, int tiles, cudaStream_t st) {
         attr[dev] = true;
     }
     const int grid = std::min(tiles, sm_count() * kStageBlocksPerSM);
-    return launch_dep(k_step_staged<S, LES, BETA, ONE, N, ADDR>, grid, kStageThreads, Tile<S>::SMEM, st, a, tiles);
+    return launch_dep(dep, k_step_staged<S, LES, BETA, ONE, N, ADDR>, grid, kStageThreads, Tile<S>::SMEM, st, a, tiles);
 }
 
 // Beta steps whose lattices all span fewer than 2^32 population elements
@@ -399,7 +399,7 @@ static int launch_staged_w(const StepArgs<N> &a, int tiles, cudaStream_t st) {
 // table of the 19 offsets when the lattices share their shape (domains and
 // single lattices), else computed per lattice (ensembles).
 template <typename S, bool LES, bool BETA, bool ONE, int N = kParamLattices>
-static int launch_staged_one(const StepArgs<N> &a, int tiles, cudaStream_t st) {
+static int launch_staged_one(const StepArgs<N> &a, int tiles, Dep dep, cudaStream_t st) {
     if constexpr (BETA) {
         bool w32 = true, same = true;
         for (int i = 0; i < a.ntab; i++) {
@@ -414,20 +414,20 @@ static int launch_staged_one(const StepArgs<N> &a, int tiles, cudaStream_t st) {
                 for (int i = 0; i < 19; i++)
                     b.koff[i] = (uint32_t)i * (uint32_t)a.tab[0].pstride + (uint32_t)dir_x(i) +
                                 (uint32_t)dir_y(i) * nx + (uint32_t)dir_z(i) * sl;
-                return launch_staged_w<S, LES, BETA, ONE, N, kAddrTab>(b, tiles, st);
+                return launch_staged_w<S, LES, BETA, ONE, N, kAddrTab>(b, tiles, dep, st);
             }
         } else {
             (void)same;
-            if (w32) return launch_staged_w<S, LES, BETA, ONE, N, kAddr32>(a, tiles, st);
+            if (w32) return launch_staged_w<S, LES, BETA, ONE, N, kAddr32>(a, tiles, dep, st);
         }
     }
-    return launch_staged_w<S, LES, BETA, ONE, N, kAddr64>(a, tiles, st);
+    return launch_staged_w<S, LES, BETA, ONE, N, kAddr64>(a, tiles, dep, st);
 }
 
 template <typename S, bool LES, bool BETA>
 static int launch_staged_k(const DomainArgs &a, int tiles, cudaStream_t st) {
-    return a.ntab == 1 ? launch_staged_one<S, LES, BETA, true>(a, tiles, st)
-                       : launch_staged_one<S, LES, BETA, false>(a, tiles, st);
+    return a.ntab == 1 ? launch_staged_one<S, LES, BETA, true>(a, tiles, Dep{}, st)
+                       : launch_staged_one<S, LES, BETA, false>(a, tiles, Dep{}, st);
 }
 
 template <typename S>
@@ -448,21 +448,21 @@ int staged_cells(int storage) {
 }
 
 template <typename S>
-static int launch_staged_batch_t(bool beta, bool les, const BatchArgs &a, int tiles, cudaStream_t st) {
+static int launch_staged_batch_t(bool beta, bool les, const BatchArgs &a, int tiles, Dep dep, cudaStream_t st) {
     if (tiles <= 0) return 0;
     if (beta)
-        return les ? launch_staged_one<S, true, true, false, kBatchLattices>(a, tiles, st)
-                   : launch_staged_one<S, false, true, false, kBatchLattices>(a, tiles, st);
-    return les ? launch_staged_one<S, true, false, false, kBatchLattices>(a, tiles, st)
-               : launch_staged_one<S, false, false, false, kBatchLattices>(a, tiles, st);
+        return les ? launch_staged_one<S, true, true, false, kBatchLattices>(a, tiles, dep, st)
+                   : launch_staged_one<S, false, true, false, kBatchLattices>(a, tiles, dep, st);
+    return les ? launch_staged_one<S, true, false, false, kBatchLattices>(a, tiles, dep, st)
+               : launch_staged_one<S, false, false, false, kBatchLattices>(a, tiles, dep, st);
 }
 
-int launch_staged_batch(int storage, bool beta, bool les, const BatchArgs &a, int tiles, cudaStream_t st) {
+int launch_staged_batch(int storage, bool beta, bool les, const BatchArgs &a, int tiles, Dep dep, cudaStream_t st) {
     switch (storage) {
-        case kF32: return launch_staged_batch_t<float>(beta, les, a, tiles, st);
-        case kF16: return launch_staged_batch_t<__half>(beta, les, a, tiles, st);
-        case kBF16: return launch_staged_batch_t<__nv_bfloat16>(beta, les, a, tiles, st);
-        case kC16: return launch_staged_batch_t<c16_t>(beta, les, a, tiles, st);
+        case kF32: return launch_staged_batch_t<float>(beta, les, a, tiles, dep, st);
+        case kF16: return launch_staged_batch_t<__half>(beta, les, a, tiles, dep, st);
+        case kBF16: return launch_staged_batch_t<__nv_bfloat16>(beta, les, a, tiles, dep, st);
+        case kC16: return launch_staged_batch_t<c16_t>(beta, les, a, tiles, dep, st);
     }
     return fail("the staged kernels take float, half or bfloat16 storage");
 }
@@ -486,7 +486,7 @@ int launch_step(int storage, int shape, int parity, bool les, const LatDesc *hta
         int units = 0;
         for (int i = 0; i < a.ntab; i++) {
             a.tab[i] = htab[c0 + i];
-            a.tab[i].first_block = units;
+            a.tab[i].first_block = a.first[i] = units;
             a.tab[i].nblocks = (int)((a.tab[i].n + per - 1) / per);
             units += a.tab[i].nblocks;
         }
@@ -566,7 +566,7 @@ static int launch_halo_param(const HaloDesc *hd, int n, int64_t max_cells, int m
     HaloArgs<N> a;
     memset(&a, 0, sizeof(a));
     memcpy(a.h, hd, (size_t)n * sizeof(HaloDesc));
-    return launch_dep(k_halo_batch<E, N>, halo_grid(max_cells, max_planes, n), kBlock, 0, st, a);
+    return launch_dep(Dep{}, k_halo_batch<E, N>, halo_grid(max_cells, max_planes, n), kBlock, 0, st, a);
 }
 
 template <typename E>
@@ -589,6 +589,68 @@ int launch_halo_batch(int storage, const HaloDesc *hd, int nd, int64_t max_cells
         case 4: return launch_halo_chunks<uint32_t>(hd, nd, max_cells, max_planes, st);
         default: return launch_halo_chunks<uint64_t>(hd, nd, max_cells, max_planes, st);
     }
+}
+}  // namespace lbm_rt
+
+namespace lbm_rt {
+// A lattice without its fields; null (and the error set) if it cannot exist.
+static lbm_lattice *new_lattice(int nx, int ny, int nz, int storage, int store_velocity, int store_density) {
+    if (nx < 3 || ny < 3 || nz < 3) {
+        fail("each lattice dimension must be at least 3");
+        return nullptr;
+    }
+    if (storage < kF32 || storage > kC16) {
+        fail("unknown storage type");
+        return nullptr;
+    }
+    const int64_t n = (int64_t)nx * ny * nz;
+    if (n > ((int64_t)1 << 31) - 1) {
+        fail("lattice has more than 2^31-1 cells");
+        return nullptr;
+    }
+    lbm_lattice *l = new lbm_lattice();
+    l->nx = nx; l->ny = ny; l->nz = nz;
+    l->n = n;
+    l->pstride = round_up(n, 256 / (int64_t)storage_bytes(storage));
+    l->storage = storage;
+    l->store_v = store_velocity ? 1 : 0;
+    l->store_rho = store_density ? 1 : 0;
+    return l;
+}
+
+static void set_fields(lbm_lattice *l) {
+    LatDesc &h = l->h;
+    h.dd = l->dd; h.flags = l->flags; h.vel = l->vel; h.rho = l->rho;
+    h.pstride = l->pstride; h.n = l->n;
+    h.nx = l->nx; h.ny = l->ny; h.nz = l->nz;
+    h.first_block = 0;
+    h.nblocks = grid_for(l->n);
+    lbm_params p{};
+    p.inv_tau = 1.0 / 0.953575;  // reference default tau (src/CLbmSkeleton.hpp:142)
+    p.tau0 = 0.953575;
+    set_params_desc(h, l->storage, p);
+}
+
+size_t lattice_block_bytes(int nx, int ny, int nz, int storage, int store_v) {
+    const int64_t n = (int64_t)nx * ny * nz, ps = round_up(n, 256 / (int64_t)storage_bytes(storage));
+    return (size_t)ps * 19 * storage_bytes(storage) + (size_t)round_up(n, 256) +
+           (store_v ? (size_t)n * 3 * real_bytes(storage) : 0);
+}
+
+int lattice_in_block(int nx, int ny, int nz, int storage, int store_v, void *block, lbm_lattice **out) {
+    *out = nullptr;
+    lbm_lattice *l = new_lattice(nx, ny, nz, storage, store_v, 0);
+    if (!l) return -1;
+    char *p = (char *)block;  // planes and flags are whole 256-byte units, so each field is aligned to one
+    l->pooled = true;
+    l->dd = p;
+    p += (size_t)l->pstride * 19 * storage_bytes(storage);
+    l->flags = (uint8_t *)p;
+    p += (size_t)round_up(l->n, 256);
+    if (l->store_v) l->vel = p;
+    set_fields(l);
+    *out = l;
+    return 0;
 }
 }  // namespace lbm_rt
 
@@ -638,21 +700,13 @@ int lbm_cu_check_wait_timeout(unsigned int polls, void *stream) {
 int lbm_cu_create(int nx, int ny, int nz, int storage, int store_velocity, int store_density, lbm_lattice **out) {
     if (!out) return fail("out is NULL");
     *out = nullptr;
-    if (nx < 3 || ny < 3 || nz < 3) return fail("each lattice dimension must be at least 3");
-    if (storage < kF32 || storage > kC16) return fail("unknown storage type");
-    const int64_t n = (int64_t)nx * ny * nz;
-    if (n > ((int64_t)1 << 31) - 1) return fail("lattice has more than 2^31-1 cells");
-    lbm_lattice *l = new lbm_lattice();
-    l->nx = nx; l->ny = ny; l->nz = nz;
-    l->n = n;
-    l->pstride = round_up(n, 256 / (int64_t)storage_bytes(storage));
-    l->storage = storage;
-    l->store_v = store_velocity ? 1 : 0;
-    l->store_rho = store_density ? 1 : 0;
+    lbm_lattice *l = new_lattice(nx, ny, nz, storage, store_velocity, store_density);
+    if (!l) return -1;
     auto cleanup = [&](const std::string &m) {
         lbm_cu_destroy(l);
         return fail(m);
     };
+    const int64_t n = l->n;
     if (cudaMalloc(&l->dd, (size_t)l->pstride * 19 * storage_bytes(storage)) != cudaSuccess)
         return cleanup("cudaMalloc of the population planes failed");
     if (cudaMalloc((void **)&l->flags, (size_t)round_up(n, 256)) != cudaSuccess) return cleanup("cudaMalloc of flags failed");
@@ -660,18 +714,7 @@ int lbm_cu_create(int nx, int ny, int nz, int storage, int store_velocity, int s
         return cleanup("cudaMalloc of velocity failed");
     if (l->store_rho && cudaMalloc(&l->rho, (size_t)n * real_bytes(storage)) != cudaSuccess)
         return cleanup("cudaMalloc of density failed");
-    if (cudaMalloc((void **)&l->d_desc, sizeof(LatDesc)) != cudaSuccess) return cleanup("cudaMalloc of descriptor failed");
-    LatDesc &h = l->h;
-    h.dd = l->dd; h.flags = l->flags; h.vel = l->vel; h.rho = l->rho;
-    h.pstride = l->pstride; h.n = n;
-    h.nx = nx; h.ny = ny; h.nz = nz;
-    h.first_block = 0;
-    h.nblocks = grid_for(n);
-    lbm_params p{};
-    p.inv_tau = 1.0 / 0.953575;  // reference default tau (src/CLbmSkeleton.hpp:142)
-    p.tau0 = 0.953575;
-    set_params_desc(h, storage, p);
-    l->dirty = true;
+    set_fields(l);
     cudaGetLastError();
     *out = l;
     return 0;
@@ -679,11 +722,12 @@ int lbm_cu_create(int nx, int ny, int nz, int storage, int store_velocity, int s
 
 int lbm_cu_destroy(lbm_lattice *l) {
     if (!l) return 0;
-    if (l->dd) cudaFree(l->dd);
-    if (l->flags) cudaFree(l->flags);
-    if (l->vel) cudaFree(l->vel);
-    if (l->rho) cudaFree(l->rho);
-    if (l->d_desc) cudaFree(l->d_desc);
+    if (!l->pooled) {
+        if (l->dd) cudaFree(l->dd);
+        if (l->flags) cudaFree(l->flags);
+        if (l->vel) cudaFree(l->vel);
+        if (l->rho) cudaFree(l->rho);
+    }
     if (l->stage) cudaFree(l->stage);
     delete l;
     return 0;
@@ -699,7 +743,6 @@ int lbm_cu_set_params(lbm_lattice *l, const lbm_params *p) {
     if (!l || !p) return fail("NULL argument");
     if (p->les_c != 0.0 && !(p->tau0 > 0.5)) return fail("the subgrid model needs tau0 > 0.5");
     set_params_desc(l->h, l->storage, *p);
-    l->dirty = true;
     return 0;
 }
 

@@ -30,8 +30,12 @@ inline cudaStream_t S(void *s) { return (cudaStream_t)s; }
 // 64^3 9.20 -> 6.90, 128^3 54.9 -> 53.1, 256^3 398.6 -> 396.1; half 24^3
 // 6.71 -> 4.94, 128^3 31.9 -> 30.5: about 2 us a launch.  Replayed from a
 // captured graph the same kernels gain nothing (24^3 4.14 -> 4.11).
+struct Dep {
+    bool on = true;  // false: an ordinary launch
+};
 template <typename... P, typename... A>
-inline int launch_dep(void (*kernel)(P...), dim3 grid, int threads, size_t shared, cudaStream_t st, const A &...args) {
+inline int launch_dep(Dep dep, void (*kernel)(P...), dim3 grid, int threads, size_t shared, cudaStream_t st,
+                      const A &...args) {
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -41,7 +45,7 @@ inline int launch_dep(void (*kernel)(P...), dim3 grid, int threads, size_t share
     cfg.dynamicSmemBytes = shared;
     cfg.stream = st;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = dep.on ? 1 : 0;
     CU(cudaLaunchKernelEx(&cfg, kernel, args...));
     return 0;
 }
@@ -79,6 +83,10 @@ int launch_step_f64_fma(int parity, bool les, const DomainArgs &a, int blocks, c
 
 // Streaming multiprocessors of the current device (cached per device).
 int sm_count();
+// A lattice's population, flag and velocity planes in one device block of
+// lattice_block_bytes (a pool's; the lattice does not free it).
+size_t lattice_block_bytes(int nx, int ny, int nz, int storage, int store_v);
+int lattice_in_block(int nx, int ny, int nz, int storage, int store_v, void *block, lbm_lattice **out);
 // Grow a lattice's staging buffer to at least `bytes`.
 int ensure_stage(lbm_lattice *l, size_t bytes);
 
@@ -95,7 +103,7 @@ int staged_cells(int storage);
 // a beta step, through the staged tiles (first_block / nblocks of the
 // descriptors count tiles of staged_cells; a beta step needs every nx a
 // multiple of 16 bytes of populations).
-int launch_staged_batch(int storage, bool beta, bool les, const BatchArgs &a, int tiles, cudaStream_t st);
+int launch_staged_batch(int storage, bool beta, bool les, const BatchArgs &a, int tiles, Dep dep, cudaStream_t st);
 // One lattice block of a checkpoint file (lbm_io.cu).
 int ckpt_write_lattice(FILE *f, lbm_lattice *l, int64_t counter);
 int ckpt_read_lattice(FILE *f, lbm_lattice *l, int64_t *counter);
@@ -111,8 +119,7 @@ struct lbm_lattice {
     void *vel = nullptr;
     void *rho = nullptr;
     lbm::LatDesc h{};
-    lbm::LatDesc *d_desc = nullptr;
-    bool dirty = true;
+    bool pooled = false;  // the fields lie in a block that the lattice's owner keeps
     void *stage = nullptr;  // staging for host copies and reduction partials
     size_t stage_bytes = 0;
     int shape = 0;  // requested kernel shape (0: per storage type, see effective_shape)
