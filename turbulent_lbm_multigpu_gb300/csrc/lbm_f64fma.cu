@@ -24,7 +24,7 @@ static_assert(sizeof(F64Fma) == sizeof(double), "same layout as double populatio
 
 template <> struct Store<F64Fma> {
     using R = double;
-    static constexpr bool kDev = false;
+    static constexpr int kDev = 0;
     __device__ static __forceinline__ R ld(const F64Fma *p, R) { return p->v; }
     __device__ static __forceinline__ void st(F64Fma *p, R v, R) { p->v = v; }
 };
