@@ -124,10 +124,11 @@ int lbm_cu_step(lbm_lattice *lat, int parity, void *stream);
  * arithmetic type is float and nx is even, else 1.  3: persistent blocks
  * that stream tiles of cells through shared memory with TMA bulk copies (a
  * producer warp keeps the next tiles in flight while eight warps compute);
- * float and the 16-bit storage types, else 1; the beta step of a lattice whose
- * nx is not a multiple of 16 bytes of populations runs shape 1.  0
- * (default): 3 for the 16-bit storage types, 1 for float and double, the
- * fastest measured on GB300.  All shapes give bit-identical results.  No
+ * float and the 16-bit storage types, else 1; the beta step of a float lattice
+ * whose nx is not a multiple of 4 runs shape 1.  0 (default): 3 for the 16-bit
+ * storage types where a launch covers 1.25 Mi cells or more (its alpha step
+ * from 0.75 Mi, its beta step from 2.25 Mi if nx is not a multiple of 8), else
+ * 1, the fastest measured on GB300.  All shapes give bit-identical results.  No
  * reference counterpart (the reference's work-group size list,
  * src/CLbmSolver.hpp:279-312, tunes its OpenCL launch instead). */
 int lbm_cu_set_kernel_shape(lbm_lattice *lat, int cells_per_thread);
@@ -348,9 +349,10 @@ int lbm_cu_batch_create(const lbm_cavity *cavities, int count, int store_velocit
 int lbm_cu_batch_destroy(lbm_batch *b);
 int lbm_cu_batch_reset(lbm_batch *b, void *stream);
 /* Ensemble kernel shape: 1 one cell per thread (default), 2 two cells per
- * thread (cavities with even nx), 3 as 1 but the alpha steps of half and
- * bfloat16 cavities run the staged tiles when every member of a launch is
- * at an alpha step.  Results are the same for every shape. */
+ * thread (cavities with even nx), 3 as 1 but the cavities of a 16-bit storage
+ * type run the staged tiles when every member of a launch is at the same kind
+ * of step and it is as large as shape 0 of a lattice asks for.  Results are
+ * the same for every shape. */
 int lbm_cu_batch_set_kernel_shape(lbm_batch *b, int cells_per_thread);
 /* Autotuner: times `trial_steps` steps of the whole ensemble for each kernel
  * shape (1, 2, 3), keeps the fastest, and resets. */

@@ -4,11 +4,11 @@
 // parameters, storage types and step counts, each with its own step
 // counter.  A tick advances every active cavity by k steps with one launch
 // per storage group and step (k_step / k_step2: each block reads its
-// cavity's parity from the descriptor table), pairs of steps replayed from a
-// captured CUDA graph.  With kernel shape 3 a chunk of 16-bit cavities whose
-// members are all at an alpha step runs the staged-tile kernel instead, and
-// so do beta steps of the cavities whose rows are whole 16-byte units (they
-// form their own groups).  The static batch (lbm_cu_batch_*) runs a fixed
+// cavity's parity from the descriptor table), without waiting for the GPU;
+// small ensembles replay pairs of steps from a captured CUDA graph.  With
+// kernel shape 3 a chunk of 16-bit cavities whose members are all at the same
+// kind of step runs the staged-tile kernel instead, if it is large enough
+// (staged_pays).  The static batch (lbm_cu_batch_*) runs a fixed
 // ensemble to completion; the server (lbm_cu_server_*) admits queued solves
 // between ticks under an HBM budget and retires finished ones (continuous
 // batching).  Results of a cavity do not depend on the other members of its
@@ -143,14 +143,15 @@ struct Ensemble {
         std::unique_ptr<BatchArgs> sargs;  // the same numbered in staged tiles (staged groups)
         int blocks = 0;
         int tiles = 0;
+        int64_t cells = 0;
+        bool ragged = false;  // some row is not whole 16-byte units of half populations
         int parities = 0;  // bit p: some member's step counter has parity p
         bool les = false;
     };
     struct Group {
         int storage = 0;
         bool pair = false;
-        bool staged = false;  // alpha steps through the staged tiles (shape 3, 16-bit storage)
-        bool aligned = false;  // staged, and every nx a multiple of 16 bytes: beta steps staged too
+        bool staged = false;  // through the staged tiles where they apply (shape 3, 16-bit storage)
         std::vector<int> members;
         std::vector<Chunk> chunks;
     };
@@ -182,17 +183,15 @@ struct Ensemble {
             const bool pair = shape == 2 && s.spec.storage != LBM_F64 && !(s.spec.nx & 1);
             const bool staged =
                 shape == 3 && (s.spec.storage == LBM_F16 || s.spec.storage == LBM_BF16 || s.spec.storage == LBM_C16);
-            const bool aligned = staged && ((int64_t)s.spec.nx * storage_bytes(s.spec.storage)) % 16 == 0;
             Group *g = nullptr;
             for (auto &x : groups)
-                if (x.storage == s.spec.storage && x.pair == pair && x.aligned == aligned) g = &x;
+                if (x.storage == s.spec.storage && x.pair == pair) g = &x;
             if (!g) {
                 groups.emplace_back();
                 g = &groups.back();
                 g->storage = s.spec.storage;
                 g->pair = pair;
                 g->staged = staged;
-                g->aligned = aligned;
             }
             g->members.push_back((int)i);
         }
@@ -225,6 +224,8 @@ struct Ensemble {
                 if (g.staged) memset(ch.sargs.get(), 0, sizeof(BatchArgs));
                 ch.les = false;
                 ch.parities = 0;
+                ch.cells = 0;
+                ch.ragged = false;
                 for (size_t k = k0; k < k1; k++) {
                     const Slot &s = slots[g.members[k]];
                     LatDesc h = s.lat->h;
@@ -232,6 +233,8 @@ struct Ensemble {
                     h.nblocks = (int)((h.n + per - 1) / per);
                     h.parity = (int)(s.done & 1);
                     first += h.nblocks;
+                    ch.cells += h.n;
+                    ch.ragged = ch.ragged || h.nx % 8;
                     if (uses_les(h)) ch.les = true;
                     a.tab[k - k0] = h;
                     a.first[k - k0] = h.first_block;
@@ -261,7 +264,7 @@ struct Ensemble {
             for (auto &ch : g.chunks) {
                 const bool all_alpha = ch.parities == 1 << ((j + 1) & 1);
                 const bool all_beta = ch.parities == 1 << (j & 1);
-                if (g.staged && (all_alpha || (all_beta && g.aligned))) {
+                if (g.staged && (all_alpha || all_beta) && staged_pays(all_beta, ch.ragged, ch.cells)) {
                     // every member at the same kind of step: staged tiles
                     ch.sargs->store_v = store ? store_v : 0;
                     ch.sargs->store_rho = 0;
@@ -573,7 +576,7 @@ int lbm_cu_server_create(double hbm_budget_bytes, int max_active, int store_velo
     s->budget = hbm_budget_bytes;
     s->max_active = max_active > 0 ? max_active : 1 << 30;
     s->e.store_v = store_velocity ? 1 : 0;
-    s->e.shape = 3;  // staged alpha steps for parity-uniform 16-bit launches (measured the faster)
+    s->e.shape = 3;  // staged tiles for large parity-uniform 16-bit launches (measured the faster)
     *out = s;
     return 0;
 }

@@ -262,7 +262,6 @@ static_assert(sizeof(HaloArgs<kHaloParam>) <= 32764, "halo descriptors exceed th
 
 template <typename E, int N>
 __global__ void k_halo_batch(const __grid_constant__ HaloArgs<N> a) {
-    follow_previous_grid();
     halo_elem<E>(a.h[blockIdx.z]);
 }
 
@@ -319,9 +318,9 @@ __global__ void __launch_bounds__(kBlock) k_dev_stats(LatDesc d, unsigned long l
 
 // ------------------------------------------------------------- dispatchers
 template <typename S, bool PAIR>
-int launch_step_t(int parity, bool les, const DomainArgs &a, int blocks, cudaStream_t st) {
+int launch_step_t(int parity, bool les, const DomainArgs &a, int blocks, Dep dep, cudaStream_t st) {
     if (blocks <= 0) return 0;
-#define STEP(K_) (les ? launch_dep(Dep{}, K_<S, true>, blocks, kBlock, 0, st, a) : launch_dep(Dep{}, K_<S, false>, blocks, kBlock, 0, st, a))
+#define STEP(K_) (les ? launch_dep(dep, K_<S, true>, blocks, kBlock, 0, st, a) : launch_dep(dep, K_<S, false>, blocks, kBlock, 0, st, a))
     if constexpr (PAIR) return parity ? STEP(k_alpha2) : STEP(k_beta2);
     else return parity ? STEP(k_alpha) : STEP(k_beta);
 #undef STEP
@@ -337,29 +336,38 @@ bool pair_shape(int storage, const LatDesc *tab, int ntab) {
 }
 
 int effective_shape(int storage, int shape, const LatDesc *tab, int ntab) {
-    if (shape == 0) shape = (storage == kF16 || storage == kBF16 || storage == kC16) ? 3 : 1;  // the measured best per storage
+    if (shape == 0) {
+        if (storage_bytes(storage) != 2) return 1;
+        int64_t cells = 0;
+        bool ragged = false;
+        for (int i = 0; i < std::min(ntab, kParamLattices); i++) {
+            cells += tab[i].n;
+            ragged = ragged || tab[i].nx % 8;
+        }
+        return staged_pays(true, ragged, cells) ? 3 : staged_pays(false, ragged, cells) ? kShapeStagedAlpha : 1;
+    }
     if (shape == 2 && pair_shape(storage, tab, ntab)) return 2;
     if (shape == 3 && storage != kF64) return 3;
     return 1;
 }
 
-static int launch_chunk(int storage, bool pair, int parity, bool les, const DomainArgs &a, int blocks,
+static int launch_chunk(int storage, bool pair, int parity, bool les, const DomainArgs &a, int blocks, Dep dep,
                         cudaStream_t st) {
     if (pair) {
         switch (storage) {
-            case kF32: return launch_step_t<float, true>(parity, les, a, blocks, st);
-            case kF16: return launch_step_t<__half, true>(parity, les, a, blocks, st);
-            case kBF16: return launch_step_t<__nv_bfloat16, true>(parity, les, a, blocks, st);
-            case kC16: return launch_step_t<c16_t, true>(parity, les, a, blocks, st);
+            case kF32: return launch_step_t<float, true>(parity, les, a, blocks, dep, st);
+            case kF16: return launch_step_t<__half, true>(parity, les, a, blocks, dep, st);
+            case kBF16: return launch_step_t<__nv_bfloat16, true>(parity, les, a, blocks, dep, st);
+            case kC16: return launch_step_t<c16_t, true>(parity, les, a, blocks, dep, st);
         }
         return fail("the two-cell kernels need a float arithmetic type");
     }
     switch (storage) {
-        case kF32: return launch_step_t<float, false>(parity, les, a, blocks, st);
-        case kF64: return launch_step_t<double, false>(parity, les, a, blocks, st);
-        case kF16: return launch_step_t<__half, false>(parity, les, a, blocks, st);
-        case kBF16: return launch_step_t<__nv_bfloat16, false>(parity, les, a, blocks, st);
-        case kC16: return launch_step_t<c16_t, false>(parity, les, a, blocks, st);
+        case kF32: return launch_step_t<float, false>(parity, les, a, blocks, dep, st);
+        case kF64: return launch_step_t<double, false>(parity, les, a, blocks, dep, st);
+        case kF16: return launch_step_t<__half, false>(parity, les, a, blocks, dep, st);
+        case kBF16: return launch_step_t<__nv_bfloat16, false>(parity, les, a, blocks, dep, st);
+        case kC16: return launch_step_t<c16_t, false>(parity, les, a, blocks, dep, st);
     }
     return fail("unknown storage type");
 }
@@ -377,7 +385,7 @@ int sm_count() {
     return cache[dev];
 }
 
-template <typename S, bool LES, bool BETA, bool ONE, int N, int ADDR>
+template <typename S, bool LES, bool BETA, bool ONE, int N, int ADDR, bool ROWS>
 static int launch_staged_w(const StepArgs<N> &a, int tiles, Dep dep, cudaStream_t st) {
     // the ring exceeds the default 48 KB of dynamic shared memory; the limit
     // is raised once per device
@@ -386,55 +394,69 @@ static int launch_staged_w(const StepArgs<N> &a, int tiles, Dep dep, cudaStream_
     CU(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) return fail("device index out of range");
     if (!attr[dev]) {
-        CU(cudaFuncSetAttribute(k_step_staged<S, LES, BETA, ONE, N, ADDR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                Tile<S>::SMEM));
+        CU(cudaFuncSetAttribute(k_step_staged<S, LES, BETA, ONE, N, ADDR, ROWS>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<S>::SMEM));
         attr[dev] = true;
     }
     const int grid = std::min(tiles, sm_count() * kStageBlocksPerSM);
-    return launch_dep(dep, k_step_staged<S, LES, BETA, ONE, N, ADDR>, grid, kStageThreads, Tile<S>::SMEM, st, a, tiles);
+    return launch_dep(dep, k_step_staged<S, LES, BETA, ONE, N, ADDR, ROWS>, grid, kStageThreads, Tile<S>::SMEM, st, a,
+                      tiles);
 }
 
 // Beta steps whose lattices all span fewer than 2^32 population elements
 // form their scatter addresses in 32-bit arithmetic (scatter_ptr): from a
-// table of the 19 offsets when the lattices share their shape (domains and
-// single lattices), else computed per lattice (ensembles).
+// table of the 19 offsets in the launch parameters when the lattices share
+// their shape (domains and single lattices), else from the tile's table where
+// there is one, else computed per lattice (ensembles).
+template <typename S, bool LES, bool ONE, int N, bool ROWS>
+static int launch_staged_beta(const StepArgs<N> &a, int tiles, Dep dep, cudaStream_t st) {
+    bool w32 = true, same = true;
+    for (int i = 0; i < a.ntab; i++) {
+        if (19 * a.tab[i].pstride >= ((int64_t)1 << 32)) w32 = false;
+        if (a.tab[i].nx != a.tab[0].nx || a.tab[i].ny != a.tab[0].ny || a.tab[i].pstride != a.tab[0].pstride)
+            same = false;
+    }
+    if constexpr (N == kParamLattices) {
+        if (w32 && same) {
+            StepArgs<N> b = a;
+            const uint32_t nx = (uint32_t)a.tab[0].nx, sl = nx * (uint32_t)a.tab[0].ny;
+            for (int i = 0; i < 19; i++)
+                b.koff[i] = (uint32_t)i * (uint32_t)a.tab[0].pstride + (uint32_t)dir_x(i) +
+                            (uint32_t)dir_y(i) * nx + (uint32_t)dir_z(i) * sl;
+            return launch_staged_w<S, LES, true, ONE, N, kAddrTab, ROWS>(b, tiles, dep, st);
+        }
+    } else {
+        (void)same;
+        if (w32) return launch_staged_w<S, LES, true, ONE, N, ROWS ? kAddr32 : kAddrTile, ROWS>(a, tiles, dep, st);
+    }
+    return launch_staged_w<S, LES, true, ONE, N, kAddr64, ROWS>(a, tiles, dep, st);
+}
+
 template <typename S, bool LES, bool BETA, bool ONE, int N = kParamLattices>
 static int launch_staged_one(const StepArgs<N> &a, int tiles, Dep dep, cudaStream_t st) {
     if constexpr (BETA) {
-        bool w32 = true, same = true;
-        for (int i = 0; i < a.ntab; i++) {
-            if (19 * a.tab[i].pstride >= ((int64_t)1 << 32)) w32 = false;
-            if (a.tab[i].nx != a.tab[0].nx || a.tab[i].ny != a.tab[0].ny || a.tab[i].pstride != a.tab[0].pstride)
-                same = false;
+        if constexpr (sizeof(S) == 2) {
+            for (int i = 0; i < a.ntab; i++)
+                if (a.tab[i].nx % Tile<S>::A) return launch_staged_beta<S, LES, ONE, N, false>(a, tiles, dep, st);
         }
-        if constexpr (N == kParamLattices) {
-            if (w32 && same) {
-                StepArgs<N> b = a;
-                const uint32_t nx = (uint32_t)a.tab[0].nx, sl = nx * (uint32_t)a.tab[0].ny;
-                for (int i = 0; i < 19; i++)
-                    b.koff[i] = (uint32_t)i * (uint32_t)a.tab[0].pstride + (uint32_t)dir_x(i) +
-                                (uint32_t)dir_y(i) * nx + (uint32_t)dir_z(i) * sl;
-                return launch_staged_w<S, LES, BETA, ONE, N, kAddrTab>(b, tiles, dep, st);
-            }
-        } else {
-            (void)same;
-            if (w32) return launch_staged_w<S, LES, BETA, ONE, N, kAddr32>(a, tiles, dep, st);
-        }
+        return launch_staged_beta<S, LES, ONE, N, true>(a, tiles, dep, st);
+    } else {
+        return launch_staged_w<S, LES, false, ONE, N, kAddr64, true>(a, tiles, dep, st);
     }
-    return launch_staged_w<S, LES, BETA, ONE, N, kAddr64>(a, tiles, dep, st);
 }
 
 template <typename S, bool LES, bool BETA>
-static int launch_staged_k(const DomainArgs &a, int tiles, cudaStream_t st) {
-    return a.ntab == 1 ? launch_staged_one<S, LES, BETA, true>(a, tiles, Dep{}, st)
-                       : launch_staged_one<S, LES, BETA, false>(a, tiles, Dep{}, st);
+static int launch_staged_k(const DomainArgs &a, int tiles, Dep dep, cudaStream_t st) {
+    return a.ntab == 1 ? launch_staged_one<S, LES, BETA, true>(a, tiles, dep, st)
+                       : launch_staged_one<S, LES, BETA, false>(a, tiles, dep, st);
 }
 
 template <typename S>
-static int launch_staged_t(int parity, bool les, const DomainArgs &a, int tiles, cudaStream_t st) {
+static int launch_staged_t(int parity, bool les, const DomainArgs &a, int tiles, Dep dep, cudaStream_t st) {
     if (tiles <= 0) return 0;
-    if (parity) return les ? launch_staged_k<S, true, false>(a, tiles, st) : launch_staged_k<S, false, false>(a, tiles, st);
-    return les ? launch_staged_k<S, true, true>(a, tiles, st) : launch_staged_k<S, false, true>(a, tiles, st);
+    if (parity)
+        return les ? launch_staged_k<S, true, false>(a, tiles, dep, st) : launch_staged_k<S, false, false>(a, tiles, dep, st);
+    return les ? launch_staged_k<S, true, true>(a, tiles, dep, st) : launch_staged_k<S, false, true>(a, tiles, dep, st);
 }
 
 int staged_cells(int storage) {
@@ -468,11 +490,11 @@ int launch_staged_batch(int storage, bool beta, bool les, const BatchArgs &a, in
 }
 
 int launch_step(int storage, int shape, int parity, bool les, const LatDesc *htab, int ntab, int sv, int sr,
-                cudaStream_t st) {
-    // the staged beta needs rows of whole 16-byte units (nx a multiple of 4
-    // float or 8 half populations)
-    bool staged = shape == 3 && storage != kF64;
-    if (staged && parity == 0)
+                Dep dep, cudaStream_t st) {
+    // the staged beta of float populations needs rows of whole 16-byte units
+    // (nx a multiple of 4)
+    bool staged = (shape == 3 && storage != kF64) || (shape == kShapeStagedAlpha && parity == 1);
+    if (staged && parity == 0 && storage == kF32)
         for (int i = 0; i < ntab; i++)
             if ((htab[i].nx * storage_bytes(storage)) % 16) staged = false;
     const bool pair = shape == 2;
@@ -506,16 +528,16 @@ int launch_step(int storage, int shape, int parity, bool les, const LatDesc *hta
         a.interleave = inter && push ? 1 : 0;
         int rc;
         if (shape == kShapeF64Fma && storage == kF64) {
-            rc = launch_step_f64_fma(parity, les, a, units, st);
+            rc = launch_step_f64_fma(parity, les, a, units, dep, st);
         } else if (staged) {
             switch (storage) {
-                case kF32: rc = launch_staged_t<float>(parity, les, a, units, st); break;
-                case kF16: rc = launch_staged_t<__half>(parity, les, a, units, st); break;
-                case kBF16: rc = launch_staged_t<__nv_bfloat16>(parity, les, a, units, st); break;
-                default: rc = launch_staged_t<c16_t>(parity, les, a, units, st); break;
+                case kF32: rc = launch_staged_t<float>(parity, les, a, units, dep, st); break;
+                case kF16: rc = launch_staged_t<__half>(parity, les, a, units, dep, st); break;
+                case kBF16: rc = launch_staged_t<__nv_bfloat16>(parity, les, a, units, dep, st); break;
+                default: rc = launch_staged_t<c16_t>(parity, les, a, units, dep, st); break;
             }
         } else {
-            rc = launch_chunk(storage, pair, parity, les, a, units, st);
+            rc = launch_chunk(storage, pair, parity, les, a, units, dep, st);
         }
         if (rc) return -1;
     }
@@ -526,7 +548,7 @@ int step_lattice(const lbm_lattice *l, int parity, bool store, cudaStream_t st) 
     const LatDesc &h = l->h;
     const int shape = l->fma64 && l->storage == kF64 ? kShapeF64Fma : effective_shape(l->storage, l->shape, &h, 1);
     return launch_step(l->storage, shape, parity & 1, uses_les(h), &h, 1, store ? l->store_v : 0,
-                       store ? l->store_rho : 0, st);
+                       store ? l->store_rho : 0, Dep{}, st);
 }
 
 Box make_box(const lbm_lattice *l, const int o[3], const int s[3]) {
@@ -566,7 +588,9 @@ static int launch_halo_param(const HaloDesc *hd, int n, int64_t max_cells, int m
     HaloArgs<N> a;
     memset(&a, 0, sizeof(a));
     memcpy(a.h, hd, (size_t)n * sizeof(HaloDesc));
-    return launch_dep(Dep{}, k_halo_batch<E, N>, halo_grid(max_cells, max_planes, n), kBlock, 0, st, a);
+    k_halo_batch<E, N><<<halo_grid(max_cells, max_planes, n), kBlock, 0, st>>>(a);
+    CU(cudaGetLastError());
+    return 0;
 }
 
 template <typename E>
@@ -1105,12 +1129,15 @@ int domain_record(lbm_domain *D, cudaStream_t st, cudaEvent_t *out) {
     return 0;
 }
 
-int domain_one_step(lbm_domain *D, int parity, cudaStream_t st, bool store, bool timed) {
+// dep: programmatic dependence on the launch before (a lone lattice's steps
+// launched one by one; with exchange launches in between, or captured into a
+// graph, it costs: half 128x120x110 in 2x2x1 subdomains 32.9 -> 41.9 us a step).
+int domain_one_step(lbm_domain *D, int parity, cudaStream_t st, bool store, bool timed, Dep dep) {
     const bool les = uses_les(D->subs[0]->h);
     const int sv = store ? D->store_v : 0, sr = store ? D->store_rho : 0;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (timed && domain_record(D, st, &e0)) return -1;
-    if (launch_step(D->storage, D->eff_shape, parity, les, D->h_tab.data(), (int)D->subs.size(), sv, sr, st))
+    if (launch_step(D->storage, D->eff_shape, parity, les, D->h_tab.data(), (int)D->subs.size(), sv, sr, dep, st))
         return -1;
     if (timed && domain_record(D, st, &e1)) return -1;
     if (timed) {
@@ -1342,7 +1369,7 @@ int lbm_cu_domain_prepare_timed_run(lbm_domain *D, int steps, int every, void *s
         const bool timed = timed_step(k, every);
         if (timed) ok = cudaEventRecordWithFlags(D->tev[2 * k], D->cap_stream, cudaEventRecordExternal) == cudaSuccess;
         ok = ok && !launch_step(D->storage, D->eff_shape, parity, les, D->h_tab.data(), (int)D->subs.size(), sv, sr,
-                                D->cap_stream);
+                                Dep{false}, D->cap_stream);
         if (timed)
             ok = ok && cudaEventRecordWithFlags(D->tev[2 * k + 1], D->cap_stream, cudaEventRecordExternal) == cudaSuccess;
         for (int a = 0; a < 3 && ok; a++)
@@ -1386,7 +1413,9 @@ int lbm_cu_domain_run(lbm_domain *D, int steps, int use_graph, void *stream) {
     };
     auto single = [&]() -> int {
         const bool last = done + 1 == steps;
-        if (domain_one_step(D, (int)(D->counter & 1), st, stores_on(D->counter + 1, last), D->profile)) return -1;
+        if (domain_one_step(D, (int)(D->counter & 1), st, stores_on(D->counter + 1, last), D->profile,
+                            Dep{D->subs.size() == 1 && !D->profile}))
+            return -1;
         D->counter++;
         done++;
         return 0;
@@ -1402,8 +1431,8 @@ int lbm_cu_domain_run(lbm_domain *D, int steps, int use_graph, void *stream) {
             if (!D->cap_stream) CU(cudaStreamCreateWithFlags(&D->cap_stream, cudaStreamNonBlocking));
             cudaGraph_t g = nullptr;
             CU(cudaStreamBeginCapture(D->cap_stream, cudaStreamCaptureModeThreadLocal));
-            int rc = domain_one_step(D, 0, D->cap_stream, false, false);
-            if (!rc) rc = domain_one_step(D, 1, D->cap_stream, false, false);
+            int rc = domain_one_step(D, 0, D->cap_stream, false, false, Dep{false});
+            if (!rc) rc = domain_one_step(D, 1, D->cap_stream, false, false, Dep{false});
             cudaError_t e = cudaStreamEndCapture(D->cap_stream, &g);
             if (rc) {
                 if (g) cudaGraphDestroy(g);

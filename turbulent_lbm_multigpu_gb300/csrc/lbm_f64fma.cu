@@ -31,12 +31,12 @@ template <> struct Store<F64Fma> {
 }  // namespace lbm
 
 namespace lbm_rt {
-int launch_step_f64_fma(int parity, bool les, const DomainArgs &a, int blocks, cudaStream_t st) {
+int launch_step_f64_fma(int parity, bool les, const DomainArgs &a, int blocks, Dep dep, cudaStream_t st) {
     if (blocks <= 0) return 0;
     if (parity)
-        return les ? launch_dep(Dep{}, k_alpha<F64Fma, true>, blocks, kBlock, 0, st, a)
-                   : launch_dep(Dep{}, k_alpha<F64Fma, false>, blocks, kBlock, 0, st, a);
-    return les ? launch_dep(Dep{}, k_beta<F64Fma, true>, blocks, kBlock, 0, st, a)
-               : launch_dep(Dep{}, k_beta<F64Fma, false>, blocks, kBlock, 0, st, a);
+        return les ? launch_dep(dep, k_alpha<F64Fma, true>, blocks, kBlock, 0, st, a)
+                   : launch_dep(dep, k_alpha<F64Fma, false>, blocks, kBlock, 0, st, a);
+    return les ? launch_dep(dep, k_beta<F64Fma, true>, blocks, kBlock, 0, st, a)
+               : launch_dep(dep, k_beta<F64Fma, false>, blocks, kBlock, 0, st, a);
 }
 }  // namespace lbm_rt

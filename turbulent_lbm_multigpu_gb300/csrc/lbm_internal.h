@@ -28,8 +28,8 @@ inline cudaStream_t S(void *s) { return (cudaStream_t)s; }
 // be set up while the grid before it on the stream drains.  Measured on runs
 // launched step by step (us per step, plain -> this): float 24^3 5.17 -> 3.48,
 // 64^3 9.20 -> 6.90, 128^3 54.9 -> 53.1, 256^3 398.6 -> 396.1; half 24^3
-// 6.71 -> 4.94, 128^3 31.9 -> 30.5: about 2 us a launch.  Replayed from a
-// captured graph the same kernels gain nothing (24^3 4.14 -> 4.11).
+// 6.71 -> 4.94, 128^3 31.9 -> 30.5: about 2 us a launch.  Not for captured
+// graphs or steps with exchange launches between them (domain_one_step).
 struct Dep {
     bool on = true;  // false: an ordinary launch
 };
@@ -67,19 +67,38 @@ bool pair_shape(int storage, const LatDesc *tab, int ntab);
 inline int cells_per_block(bool pair) { return pair ? kPairCells : kBlock; }
 
 // Kernel shapes of a step: 1 one cell per thread, 2 two cells per thread,
-// 3 tiles staged through shared memory by bulk copies, 0 automatic (3 for
-// the 16-bit storage types, 1 otherwise: the fastest measured on GB300).
-// The shape a set of lattices runs: 2 needs float arithmetic and even nx,
-// 3 float/half/bfloat16 storage; otherwise 1.
+// 3 tiles staged through shared memory by bulk copies, 0 automatic: for the
+// 16-bit storage types 3 where both kinds of step are the faster staged
+// (staged_pays), the staged alpha and the one-cell beta step where only the
+// alpha step is (kShapeStagedAlpha), 1 otherwise.  The shape a set of lattices runs: 2 needs
+// float arithmetic and even nx, 3 float or 16-bit storage; otherwise 1.
+//
+// Small launches do not fill the staged kernel's persistent blocks with
+// tiles, and a tile's way through the ring is longer than a load and a store.
+// Measured (half, us per step launched one by one, one-cell / staged): 24^3
+// 3.15 / 5.23, 64^3 6.16 / 8.55, 96^3 15.2 / 16.1, 112^3 (1.40 M cells) 22.7 /
+// 22.3, 128^3 33.3 / 30.9, 144^3 55.7 / 43.9, 176^3 101 / 75.6; rows that are
+// not whole 16-byte units: 121x99x87 (1.04 M) 17.4 / 18.3, 129x128x128 33.7 /
+// 32.2 (its beta kernels 41.3 / 41.8), 177x176x176 102.5 / 77.9; c16 64^3 6.76 / 8.69, 112^3 26.9 / 26.9,
+// 176^3 111 / 92.9.  The alpha kernels alone cross earlier (half, us): 64^3
+// 10.5 / 10.7, 96^3 18.6 / 17.5, 121x99x87 20.7 / 18.8.
+constexpr int64_t kStagedAlphaCells = 786432;    // alpha steps
+constexpr int64_t kStagedCells = 1310720;        // beta steps, every row whole 16-byte units
+constexpr int64_t kStagedRaggedCells = 2359296;  // beta steps, other rows
+inline bool staged_pays(bool beta, bool ragged, int64_t cells) {
+    return cells >= (!beta ? kStagedAlphaCells : ragged ? kStagedRaggedCells : kStagedCells);
+}
 int effective_shape(int storage, int shape, const LatDesc *tab, int ntab);
 
 // Internal kernel shape of double lattices that run the contracted FP64
 // kernels (lbm_cu_set_fp64_contraction): one cell per thread, fused
 // multiply-adds (lbm_f64fma.cu).
 constexpr int kShapeF64Fma = 4;
+// Internal kernel shape between 1 and 3: staged alpha, one-cell beta steps.
+constexpr int kShapeStagedAlpha = 5;
 // One step of up to kParamLattices double lattices with the contracted
 // kernels (lbm_f64fma.cu); blocks of kBlock cells.
-int launch_step_f64_fma(int parity, bool les, const DomainArgs &a, int blocks, cudaStream_t st);
+int launch_step_f64_fma(int parity, bool les, const DomainArgs &a, int blocks, Dep dep, cudaStream_t st);
 
 // Streaming multiprocessors of the current device (cached per device).
 int sm_count();
@@ -93,7 +112,7 @@ int ensure_stage(lbm_lattice *l, size_t bytes);
 // One step over `ntab` lattices of one storage type, kParamLattices
 // descriptors per launch.
 int launch_step(int storage, int shape, int parity, bool les, const LatDesc *htab, int ntab, int sv, int sr,
-                cudaStream_t st);
+                Dep dep, cudaStream_t st);
 // One step of a lattice in its own kernel shape; store: write u and rho, if
 // the lattice keeps them.
 int step_lattice(const lbm_lattice *l, int parity, bool store, cudaStream_t st);
