@@ -246,7 +246,7 @@ int lbm_cu_domain_perturb(lbm_domain *dom, uint64_t seed, double amp, void *stre
 /* `steps` calls of CController::computeNextStep for every subdomain
  * (src/CController.hpp:385-391): one batched step launch over all
  * subdomains, then the halo exchange in x, y, z order.  Whole pairs of steps
- * replay a captured CUDA graph when use_graph != 0. */
+ * of several subdomains replay a captured CUDA graph when use_graph != 0. */
 int lbm_cu_domain_run(lbm_domain *dom, int steps, int use_graph, void *stream);
 /* Velocity and density (when the domain stores them) are written on every
  * `interval`-th step, like STORE_VELOCITY / STORE_DENSITY at interval 1

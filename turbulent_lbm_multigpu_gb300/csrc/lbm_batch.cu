@@ -163,10 +163,18 @@ struct Ensemble {
     cudaGraphExec_t graph = nullptr;
     std::vector<int> graph_parity;  // parities baked into the captured graph
     cudaStream_t cap = nullptr;
+    static constexpr int kSideStreams = 3;
+    cudaStream_t side_stream[kSideStreams] = {};
+    cudaEvent_t forked = nullptr, joined[kSideStreams] = {};
 
     ~Ensemble() {
         drop_graph();
         if (cap) cudaStreamDestroy(cap);
+        for (cudaStream_t x : side_stream)
+            if (x) cudaStreamDestroy(x);
+        for (cudaEvent_t x : joined)
+            if (x) cudaEventDestroy(x);
+        if (forked) cudaEventDestroy(forked);
         for (auto &s : slots)
             if (s.lat) lbm_cu_destroy(s.lat);
     }
@@ -259,24 +267,55 @@ struct Ensemble {
         return 0;
     }
 
+    int launch_one(const Group &g, Chunk &ch, int j, bool store, Dep dep, cudaStream_t st) {
+        const bool all_alpha = ch.parities == 1 << ((j + 1) & 1);
+        const bool all_beta = ch.parities == 1 << (j & 1);
+        if (g.staged && (all_alpha || all_beta) && staged_pays(all_beta, ch.ragged, ch.cells)) {
+            // every member at the same kind of step: staged tiles
+            ch.sargs->store_v = store ? store_v : 0;
+            ch.sargs->store_rho = 0;
+            return launch_staged_batch(g.storage, all_beta, ch.les, *ch.sargs, ch.tiles, dep, st);
+        }
+        ch.args->store_v = store ? store_v : 0;
+        ch.args->store_rho = 0;
+        return launch_tick(g.storage, g.pair, ch.les, *ch.args, ch.blocks, j, all_alpha ? 1 : all_beta ? 2 : 0, dep, st);
+    }
     int launch_all(int j, bool store, Dep dep, cudaStream_t st) {
         for (auto &g : groups)
-            for (auto &ch : g.chunks) {
-                const bool all_alpha = ch.parities == 1 << ((j + 1) & 1);
-                const bool all_beta = ch.parities == 1 << (j & 1);
-                if (g.staged && (all_alpha || all_beta) && staged_pays(all_beta, ch.ragged, ch.cells)) {
-                    // every member at the same kind of step: staged tiles
-                    ch.sargs->store_v = store ? store_v : 0;
-                    ch.sargs->store_rho = 0;
-                    if (launch_staged_batch(g.storage, all_beta, ch.les, *ch.sargs, ch.tiles, dep, st)) return -1;
-                    continue;
-                }
-                ch.args->store_v = store ? store_v : 0;
-                ch.args->store_rho = 0;
-                if (launch_tick(g.storage, g.pair, ch.les, *ch.args, ch.blocks, j, all_alpha ? 1 : all_beta ? 2 : 0, dep, st))
-                    return -1;
-            }
+            for (auto &ch : g.chunks)
+                if (launch_one(g, ch, j, store, dep, st)) return -1;
         return 0;
+    }
+
+    // Steps j .. k-1 launched one by one, the last one storing u.  The chunks
+    // hold different cavities, so each runs its steps on a stream of its own
+    // between a fork from `st` and a join with it: the blocks of one fill the
+    // slots that the last blocks of another's step leave.
+    int launch_steps(int64_t j, int64_t k, cudaStream_t st) {
+        std::vector<std::pair<Group *, Chunk *>> all;
+        for (auto &g : groups)
+            for (auto &ch : g.chunks) all.push_back({&g, &ch});
+        const size_t side = std::min<size_t>(kSideStreams, all.size() - 1);
+        for (size_t q = 0; q < side; q++) {
+            if (!side_stream[q]) CU(cudaStreamCreateWithFlags(&side_stream[q], cudaStreamNonBlocking));
+            if (!joined[q]) CU(cudaEventCreateWithFlags(&joined[q], cudaEventDisableTiming));
+        }
+        if (side) {
+            if (!forked) CU(cudaEventCreateWithFlags(&forked, cudaEventDisableTiming));
+            CU(cudaEventRecord(forked, st));
+            for (size_t q = 0; q < side; q++) CU(cudaStreamWaitEvent(side_stream[q], forked, 0));
+        }
+        int rc = 0;
+        for (; j < k && !rc; j++)
+            for (size_t q = 0; q < all.size() && !rc; q++) {
+                const size_t s = q % (side + 1);
+                rc = launch_one(*all[q].first, *all[q].second, (int)(j & 1), j + 1 == k, Dep{}, s ? side_stream[s - 1] : st);
+            }
+        for (size_t q = 0; q < side; q++) {
+            CU(cudaEventRecord(joined[q], side_stream[q]));
+            CU(cudaStreamWaitEvent(st, joined[q], 0));
+        }
+        return rc;
     }
 
     int64_t active_count() const {
@@ -327,9 +366,7 @@ struct Ensemble {
             for (int64_t r = 0; r < reps; r++) CU(cudaGraphLaunch(graph, st));
             j = 2 * reps;
         }
-        for (; j < plain; j++)
-            if (launch_all((int)(j & 1), false, Dep{}, st)) return -1;
-        if (launch_all((int)((k - 1) & 1), true, Dep{}, st)) return -1;
+        if (launch_steps(j, k, st)) return -1;
         for (auto &s : slots)
             if (s.active) s.done += k;
         return 0;

@@ -1426,7 +1426,10 @@ int lbm_cu_domain_run(lbm_domain *D, int steps, int use_graph, void *stream) {
     const bool plain_pairs = (D->store_interval == 0) || (!D->store_v && !D->store_rho);
     int pairs = (steps - done) / 2;
     if (D->store_interval == 0 && (steps - done) % 2 == 0 && pairs > 0) pairs--;  // last pair stores
-    if (pairs > 0 && use_graph && plain_pairs && !D->profile) {
+    // a lone subdomain's steps follow one another faster launched one by one
+    // with programmatic dependence (float 24^3 4.1 -> 3.5 us, 64^3 8.2 -> 6.9,
+    // 128^3 54.2 -> 53.1; half 64^3 7.2 -> 6.2)
+    if (pairs > 0 && use_graph && plain_pairs && !D->profile && D->subs.size() > 1) {
         if (!D->graph) {
             if (!D->cap_stream) CU(cudaStreamCreateWithFlags(&D->cap_stream, cudaStreamNonBlocking));
             cudaGraph_t g = nullptr;
