@@ -340,8 +340,8 @@ int lbm_cu_run(lbm_lattice *lat, int64_t first_step, int64_t steps, void *stream
 /* An ensemble of cavities of different sizes, parameters, storage types and
  * step counts, all resident, advanced together: one launch per storage type
  * and step covers every unfinished cavity, every cavity stops at its own
- * step count (pairs of steps of small ensembles replay a captured CUDA graph
- * when use_graph != 0).  Each cavity's
+ * step count.  use_graph is accepted and has no effect: the steps are launched
+ * one by one, ahead of the GPU, which is faster than replaying them.  Each cavity's
  * fields are the same as when it runs alone (lbm_cu_batch_lattice gives
  * its lattice for readback; velocity is written on its last step when
  * store_velocity is set). */

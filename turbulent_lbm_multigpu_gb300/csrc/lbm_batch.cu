@@ -4,9 +4,8 @@
 // parameters, storage types and step counts, each with its own step
 // counter.  A tick advances every active cavity by k steps with one launch
 // per storage group and step (k_step / k_step2: each block reads its
-// cavity's parity from the descriptor table), without waiting for the GPU;
-// small ensembles replay pairs of steps from a captured CUDA graph.  With
-// kernel shape 3 a chunk of 16-bit cavities whose members are all at the same
+// cavity's parity from the descriptor table), without waiting for the GPU,
+// the groups on streams of their own.  With kernel shape 3 a chunk of 16-bit cavities whose members are all at the same
 // kind of step runs the staged-tile kernel instead, if it is large enough
 // (staged_pays).  The static batch (lbm_cu_batch_*) runs a fixed
 // ensemble to completion; the server (lbm_cu_server_*) admits queued solves
@@ -117,16 +116,6 @@ int cavity_reset(lbm_lattice *l, const lbm_cavity &c, cudaStream_t st) {
     return 0;
 }
 
-// Where a tick replays its pairs of steps from a graph.  Launched one by one
-// with programmatic dependent launch the steps follow one another faster on
-// the GPU, but a launch with its 31 KB of descriptors takes the host about
-// 5 us: ensembles whose steps are shorter than that are replayed.  Measured
-// (half float, half half, us per step, graph / launches): 4 cavities of 24^3
-// 9.5 / 11.4, 4 of 32^3 13.9 / 12.5, 16 of 40^3 27.9 / 25.2, 2 of 96^3 41.7 /
-// 39.4.  Capturing a pair costs as much as ten pairs' launches.
-constexpr int64_t kGraphSteps = 24;
-constexpr int64_t kGraphCells = 96 * 1024;
-
 struct Ensemble {
     struct Slot {
         lbm_cavity spec{};
@@ -143,8 +132,6 @@ struct Ensemble {
         std::unique_ptr<BatchArgs> sargs;  // the same numbered in staged tiles (staged groups)
         int blocks = 0;
         int tiles = 0;
-        int64_t cells = 0;
-        bool ragged = false;  // some row is not whole 16-byte units of half populations
         int parities = 0;  // bit p: some member's step counter has parity p
         bool les = false;
     };
@@ -153,6 +140,9 @@ struct Ensemble {
         bool pair = false;
         bool staged = false;  // through the staged tiles where they apply (shape 3, 16-bit storage)
         std::vector<int> members;
+        size_t per = 0;  // members of a chunk
+        int64_t cells = 0;
+        bool ragged = false;  // some row is not whole 16-byte units of half populations
         std::vector<Chunk> chunks;
     };
     std::vector<Slot> slots;
@@ -160,16 +150,11 @@ struct Ensemble {
     int store_v = 0;
     int shape = 1;
     bool dirty = true;
-    cudaGraphExec_t graph = nullptr;
-    std::vector<int> graph_parity;  // parities baked into the captured graph
-    cudaStream_t cap = nullptr;
     static constexpr int kSideStreams = 3;
     cudaStream_t side_stream[kSideStreams] = {};
     cudaEvent_t forked = nullptr, joined[kSideStreams] = {};
 
     ~Ensemble() {
-        drop_graph();
-        if (cap) cudaStreamDestroy(cap);
         for (cudaStream_t x : side_stream)
             if (x) cudaStreamDestroy(x);
         for (cudaEvent_t x : joined)
@@ -177,10 +162,6 @@ struct Ensemble {
         if (forked) cudaEventDestroy(forked);
         for (auto &s : slots)
             if (s.lat) lbm_cu_destroy(s.lat);
-    }
-    void drop_graph() {
-        if (graph) cudaGraphExecDestroy(graph);
-        graph = nullptr;
     }
     // Member groups of the active cavities, one per (storage, shape).
     int build_groups() {
@@ -204,36 +185,38 @@ struct Ensemble {
             g->members.push_back((int)i);
         }
         for (auto &g : groups) {
-            g.chunks.resize((g.members.size() + kBatchLattices - 1) / kBatchLattices);
+            // an ensemble of one storage type runs as two chunks, so that there
+            // are two to fill each other's last waves (20 half cavities 64.2k
+            // -> 70.4k MLUPS, 20 float ones 40.2k -> 41.0k)
+            const size_t n = g.members.size(), parts = groups.size() == 1 ? 2 : 1;
+            g.per = std::min<size_t>(kBatchLattices, (n + parts - 1) / parts);
+            g.chunks.resize((n + g.per - 1) / g.per);
             for (auto &c : g.chunks) {
                 c.args.reset(new BatchArgs());
                 if (g.staged) c.sargs.reset(new BatchArgs());
             }
         }
         dirty = false;
-        drop_graph();
         return refresh_tables();
     }
 
     // Descriptors with the current step-counter parities (and block
-    // numbering) into the launch arguments; a graph captured with other
-    // parities is dropped.
+    // numbering) into the launch arguments.
     int refresh_tables() {
-        std::vector<int> parity;
         for (auto &g : groups) {
             const int per = cells_per_block(g.pair);
+            g.cells = 0;
+            g.ragged = false;
             for (size_t c = 0; c < g.chunks.size(); c++) {
                 Chunk &ch = g.chunks[c];
                 BatchArgs &a = *ch.args;
                 memset(&a, 0, sizeof(a));
-                const size_t k0 = c * kBatchLattices, k1 = std::min(g.members.size(), k0 + kBatchLattices);
+                const size_t k0 = c * g.per, k1 = std::min(g.members.size(), k0 + g.per);
                 int first = 0, tile = 0;
                 const int tcells = g.staged ? staged_cells(g.storage) : 0;
                 if (g.staged) memset(ch.sargs.get(), 0, sizeof(BatchArgs));
                 ch.les = false;
                 ch.parities = 0;
-                ch.cells = 0;
-                ch.ragged = false;
                 for (size_t k = k0; k < k1; k++) {
                     const Slot &s = slots[g.members[k]];
                     LatDesc h = s.lat->h;
@@ -241,12 +224,11 @@ struct Ensemble {
                     h.nblocks = (int)((h.n + per - 1) / per);
                     h.parity = (int)(s.done & 1);
                     first += h.nblocks;
-                    ch.cells += h.n;
-                    ch.ragged = ch.ragged || h.nx % 8;
+                    g.cells += h.n;
+                    g.ragged = g.ragged || h.nx % 8;
                     if (uses_les(h)) ch.les = true;
                     a.tab[k - k0] = h;
                     a.first[k - k0] = h.first_block;
-                    parity.push_back(h.parity);
                     ch.parities |= 1 << h.parity;
                     if (g.staged) {
                         h.first_block = tile;
@@ -262,15 +244,13 @@ struct Ensemble {
                 ch.tiles = tile;
             }
         }
-        if (parity != graph_parity) drop_graph();
-        graph_parity = parity;
         return 0;
     }
 
     int launch_one(const Group &g, Chunk &ch, int j, bool store, Dep dep, cudaStream_t st) {
         const bool all_alpha = ch.parities == 1 << ((j + 1) & 1);
         const bool all_beta = ch.parities == 1 << (j & 1);
-        if (g.staged && (all_alpha || all_beta) && staged_pays(all_beta, ch.ragged, ch.cells)) {
+        if (g.staged && (all_alpha || all_beta) && staged_pays(all_beta, g.ragged, g.cells)) {
             // every member at the same kind of step: staged tiles
             ch.sargs->store_v = store ? store_v : 0;
             ch.sargs->store_rho = 0;
@@ -280,18 +260,16 @@ struct Ensemble {
         ch.args->store_rho = 0;
         return launch_tick(g.storage, g.pair, ch.les, *ch.args, ch.blocks, j, all_alpha ? 1 : all_beta ? 2 : 0, dep, st);
     }
-    int launch_all(int j, bool store, Dep dep, cudaStream_t st) {
-        for (auto &g : groups)
-            for (auto &ch : g.chunks)
-                if (launch_one(g, ch, j, store, dep, st)) return -1;
-        return 0;
-    }
 
-    // Steps j .. k-1 launched one by one, the last one storing u.  The chunks
+    // k steps launched one by one, the last one storing u.  The chunks
     // hold different cavities, so each runs its steps on a stream of its own
     // between a fork from `st` and a join with it: the blocks of one fill the
-    // slots that the last blocks of another's step leave.
-    int launch_steps(int64_t j, int64_t k, cudaStream_t st) {
+    // slots that the last blocks of another's step leave.  A launch with its 31
+    // KB of descriptors takes the host about 3 us.  Measured against pairs of
+    // steps replayed from a graph on one stream (half float, half half, us per
+    // step): 4 cavities of 24^3 9.5 -> 5.6, 4 of 32^3 13.9 -> 6.0, 16 of 40^3
+    // 27.9 -> 18.4, 2 of 96^3 41.7 -> 32.2.
+    int launch_steps(int64_t k, cudaStream_t st) {
         std::vector<std::pair<Group *, Chunk *>> all;
         for (auto &g : groups)
             for (auto &ch : g.chunks) all.push_back({&g, &ch});
@@ -306,7 +284,7 @@ struct Ensemble {
             for (size_t q = 0; q < side; q++) CU(cudaStreamWaitEvent(side_stream[q], forked, 0));
         }
         int rc = 0;
-        for (; j < k && !rc; j++)
+        for (int64_t j = 0; j < k && !rc; j++)
             for (size_t q = 0; q < all.size() && !rc; q++) {
                 const size_t s = q % (side + 1);
                 rc = launch_one(*all[q].first, *all[q].second, (int)(j & 1), j + 1 == k, Dep{}, s ? side_stream[s - 1] : st);
@@ -324,15 +302,8 @@ struct Ensemble {
         return n;
     }
 
-    int64_t active_cells() const {
-        int64_t n = 0;
-        for (auto &s : slots)
-            if (s.active) n += s.lat->n;
-        return n;
-    }
-
     // Advance every active cavity by k steps; the last step writes u.
-    int tick(int64_t k, bool use_graph, cudaStream_t st) {
+    int tick(int64_t k, cudaStream_t st) {
         if (k <= 0 || active_count() == 0) return 0;
         // nothing here waits for the GPU: descriptors travel with the launches
         if (dirty) {
@@ -340,33 +311,7 @@ struct Ensemble {
         } else if (refresh_tables()) {
             return -1;
         }
-        const int64_t plain = k - 1;
-        int64_t j = 0;
-        if (use_graph && plain >= kGraphSteps && active_cells() < kGraphCells) {
-            if (!graph) {
-                if (!cap) CU(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
-                cudaGraph_t g = nullptr;
-                CU(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
-                int rc = launch_all(0, false, Dep{false}, cap);
-                if (!rc) rc = launch_all(1, false, Dep{false}, cap);
-                cudaError_t e = cudaStreamEndCapture(cap, &g);
-                if (rc) {
-                    if (g) cudaGraphDestroy(g);
-                    return -1;
-                }
-                if (e != cudaSuccess) return fail(std::string("graph capture: ") + cudaGetErrorString(e));
-                e = cudaGraphInstantiate(&graph, g, 0);
-                cudaGraphDestroy(g);
-                if (e != cudaSuccess) {
-                    graph = nullptr;
-                    return fail(std::string("graph instantiate: ") + cudaGetErrorString(e));
-                }
-            }
-            const int64_t reps = plain / 2;
-            for (int64_t r = 0; r < reps; r++) CU(cudaGraphLaunch(graph, st));
-            j = 2 * reps;
-        }
-        if (launch_steps(j, k, st)) return -1;
+        if (launch_steps(k, st)) return -1;
         for (auto &s : slots)
             if (s.active) s.done += k;
         return 0;
@@ -538,12 +483,13 @@ int lbm_cu_batch_set_kernel_shape(lbm_batch *b, int cells_per_thread) {
 }
 
 int lbm_cu_batch_run(lbm_batch *b, int64_t max_steps, int use_graph, void *stream) {
+    (void)use_graph;
     if (!b) return fail("NULL batch");
     int64_t budget = max_steps < 0 ? INT64_MAX : max_steps;
     b->e.retire_finished();
     while (budget > 0 && b->e.active_count() > 0) {
         const int64_t k = std::min(budget, b->e.min_remaining());
-        if (b->e.tick(k, use_graph != 0, S(stream))) return -1;
+        if (b->e.tick(k, S(stream))) return -1;
         budget -= k;
         b->e.retire_finished();
     }
@@ -563,9 +509,9 @@ int lbm_cu_batch_tune(lbm_batch *b, int trial_steps, int *cells_per_thread, doub
         b->e.shape = shape;
         b->e.dirty = true;
         if (lbm_cu_batch_reset(b, stream)) return -1;
-        if (b->e.tick(2, true, st)) return -1;  // warm-up (and table build)
+        if (b->e.tick(2, st)) return -1;  // warm-up (and table build)
         CU(cudaEventRecord(e0, st));
-        if (b->e.tick(trial_steps, true, st)) return -1;
+        if (b->e.tick(trial_steps, st)) return -1;
         CU(cudaEventRecord(e1, st));
         CU(cudaEventSynchronize(e1));
         float ms = 0.f;
@@ -683,6 +629,7 @@ static int server_admit(lbm_server *s, cudaStream_t st) {
 }
 
 int lbm_cu_server_tick(lbm_server *s, int64_t max_steps, int use_graph, int *admitted, void *stream) {
+    (void)use_graph;
     if (!s) return fail("NULL server");
     cudaStream_t st = S(stream);
     const int adm = server_admit(s, st);
@@ -693,7 +640,7 @@ int lbm_cu_server_tick(lbm_server *s, int64_t max_steps, int use_graph, int *adm
         int64_t cells = 0;
         for (auto &sl : s->e.slots)
             if (sl.active) cells += sl.lat->n;
-        if (s->e.tick(k, use_graph != 0, st)) return -1;
+        if (s->e.tick(k, st)) return -1;
         s->cell_updates += cells * k;
     }
     for (auto &sl : s->e.slots)
