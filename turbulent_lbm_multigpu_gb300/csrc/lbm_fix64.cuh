@@ -18,9 +18,10 @@
 // the FP64 pipe, which works beside the integer ones.
 //
 // Measured (256^3 in 2x2x1 subdomains, subgrid model, per step): 8.39 ms ->
-// 3.00 ms (2.00k -> 5.59k MLUPS), 85 double operations per cell instead of
-// 275 (the FP64 pipe still bounds it, at about 85 % of its measured rate; the
-// shift and logic pipe is busy for 65 % of the time); 48x40x36 43 -> 21 us,
+// 3.00 ms (2.00k -> 5.60k MLUPS), 76 double operations per cell instead of
+// 275; the FP64 pipe is 65 % busy, the shift and logic pipe 72 %, so that
+// neither side has much left to take from the other (the last addition of 4
+// to 12 populations moved over here too: 3.08-3.18 ms); 48x40x36 43 -> 21 us,
 // 24^3 24 -> 17 us.
 //
 // Every step rounds as the double operation it stands for, so the results
