@@ -167,9 +167,12 @@ int lbm_cu_write(lbm_lattice *lat, int field, const int origin[3], const int siz
 int lbm_cu_halo(lbm_lattice *src, const int src_origin[3], lbm_lattice *dst, const int dst_origin[3],
                 const int size[3], const int norm[3], void *stream);
 
-/* FP64 compensated (Neumaier) sums over fluid cells of mass, momentum and
- * kinetic energy of the populations currently stored: out = {sum rho,
- * sum jx, sum jy, sum jz, sum |j|^2/2}.  `layout` 0: standard slots (after a
+/* Sums over fluid cells of mass, momentum and kinetic energy of the
+ * populations currently stored: out = {sum rho, sum jx, sum jy, sum jz,
+ * sum |j|^2/2}.  Exact, rounded to double at the end, over cells of ordinary
+ * populations (moving ones in [2^-8, 2^-3), the one at rest in [2^-8, 2^-1);
+ * double ones from 2^-9); other cells are summed in compensated (Neumaier)
+ * double arithmetic.  `layout` 0: standard slots (after a
  * beta step), 1: opposite slots (after an alpha step or the seeded start-up).
  * No reference counterpart. */
 int lbm_cu_reduce_conserved(lbm_lattice *lat, int layout, double out[5], void *stream);
@@ -177,7 +180,8 @@ int lbm_cu_reduce_conserved(lbm_lattice *lat, int layout, double out[5], void *s
 /* Velocity error of lattice a against lattice b (same size) over the fluid
  * cells of a, in FP64: out = {max |ua - ub|, sum |ua - ub|^2, sum |ub|^2,
  * max |ub|, number of cells}, u = sum_i e_i f_i of the stored populations
- * in each lattice's slot layout.  For precision studies against an FP64
+ * in each lattice's slot layout.  The sums of squares are exact over ordinary
+ * cells, as above; others are summed in double arithmetic.  For precision studies against an FP64
  * run; no reference counterpart. */
 int lbm_cu_compare_velocity(lbm_lattice *a, int layout_a, lbm_lattice *b, int layout_b, double out[5],
                             void *stream);
@@ -195,7 +199,7 @@ int lbm_cu_deviation_stats(lbm_lattice *lat, double out[5], void *stream);
  * handed out under a budget, or a monitor that must not trigger the implicit
  * synchronisation of cudaMalloc/cudaFree, cannot afford that.  This variant
  * keeps its partial sums in a fixed device array inside the library
- * (160 KB, present on every GPU that loads the library until the process
+ * (176 KB, present on every GPU that loads the library until the process
  * exits) and calls no allocator.  Limit: lattices of at most 134,217,728
  * cells (512^3); larger ones are rejected with an error.  The first call on
  * a device looks up the array's device address, so make that first call

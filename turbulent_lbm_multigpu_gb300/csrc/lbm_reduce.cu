@@ -12,8 +12,8 @@
 // (|u| below 0.3), so a float one is a whole multiple of 2^-31 and a double
 // one (from 2^-9) of 2^-61.  Cells within those bounds are summed exactly in
 // integers: moments in 32 (64) bits, squares of the momentum in 64 (128),
-// totals in 128.  The sums then do not depend on the order of the cells and
-// round once, at the end.  A cell with any population outside the bounds
+// totals in 128 and those of double cells' squares in 160 (Squares).  The sums
+// then do not depend on the order of the cells and round once, at the end.  A cell with any population outside the bounds
 // (negative, large, infinite, not a number) is summed in double arithmetic
 // with compensation, as the whole lattice was before.
 //
@@ -129,19 +129,48 @@ __device__ __forceinline__ i128 warp_max(i128 v) {
     }
     return v;
 }
-// v 2^-lsb, rounded once where v has at most 117 significant bits.
-__device__ double to_double(i128 v, int lsb) {
+__device__ __forceinline__ uint64_t warp_sum(uint64_t v) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, (unsigned long long)v, o);
+    return v;
+}
+// The double nearest to (v + low 2^-32) 2^-lsb; low only where v >= 0.
+__device__ double to_double(i128 v, int lsb, uint32_t low = 0) {
     const bool neg = v < 0;
-    const u128 m = neg ? (u128)0 - (u128)v : (u128)v;
-    const double d = scalbn((double)(uint64_t)(m >> 64), 64 - lsb) + scalbn((double)(uint64_t)m, -lsb);
+    u128 m = neg ? (u128)0 - (u128)v : (u128)v;
+    if (m >> 96) {
+        m |= low ? 1 : 0;  // far below the last place of a double
+    } else {
+        m = (m << 32) | low;
+        lsb += 32;
+    }
+    if (m == 0) return 0.0;
+    const uint64_t hi = (uint64_t)(m >> 64);
+    const int s = hi ? __clzll((long long)hi) : 64 + __clzll((long long)(uint64_t)m);
+    m <<= s;
+    // 64 leading bits, the last one set if any below is: one rounding, here
+    const double d = scalbn(__ull2double_rn((uint64_t)(m >> 64) | ((uint64_t)m ? 1u : 0u)), 64 - s - lsb);
     return neg ? -d : d;
 }
+
+// Exact total of squares in units of 2^-122 (each below 2^125): the upper 96
+// bits of each in one sum (units of 2^-90), the lower 32 in another, so that
+// 2^31 cells of any size fit and the smallest count.  LOW false: the
+// squares are whole multiples of 2^-90 (float cells).
+template <bool LOW> struct Squares {
+    i128 hi = 0;
+    uint64_t lo = 0;
+    __device__ __forceinline__ void add(u128 e) {
+        hi += (i128)(e >> 32);
+        if (LOW) lo += (uint32_t)e;
+    }
+};
 
 // Partial results of a block: five exact sums and five compensated ones
 // (cells outside the fixed-point bounds).
 struct RedPartial {
     i128 fix[5];
     Acc acc[5];
+    uint64_t low;  // of the energy's squares (Squares::lo)
 };
 // Blocks of a reduction: a few per SM; every thread walks the lattice with
 // the stride of the whole grid.
@@ -195,7 +224,10 @@ __global__ void __launch_bounds__(kBlock, 2) k_reduce(LatDesc d, int layout, Red
     constexpr int V = sizeof(R) == 4 ? 2 : 1;
     __shared__ Acc sh[5][kBlock];
     __shared__ i128 wsum[kBlock / 32][5];
+    __shared__ uint64_t wlow[kBlock / 32];
+    constexpr bool kLow = sizeof(R) == 8;
     i128 tot[5] = {0, 0, 0, 0, 0};
+    uint64_t low = 0;
     bool odd = false;  // this thread has summed a cell in double arithmetic
     for (int64_t c = V * ((int64_t)blockIdx.x * kBlock + threadIdx.x); c < d.n; c += (int64_t)V * gridDim.x * kBlock) {
         // planes and flags are padded beyond n (256 bytes): a pair may read past the last cell
@@ -217,9 +249,10 @@ __global__ void __launch_bounds__(kBlock, 2) k_reduce(LatDesc d, int layout, Red
                     for (int a = 0; a < 3; a++) e += (uint64_t)((int64_t)j[a] * j[a]);
                     tot[4] += e;
                 } else {
-                    u128 e = 0;  // units of 2^-122, kept to 2^-90
+                    u128 e = 0;  // units of 2^-122
                     for (int a = 0; a < 3; a++) e += square(j[a]);
                     tot[4] += (i128)(e >> 32);
+                    low += (uint32_t)e;
                 }
             } else {
                 if (!odd)
@@ -238,6 +271,10 @@ __global__ void __launch_bounds__(kBlock, 2) k_reduce(LatDesc d, int layout, Red
         const i128 v = warp_sum(tot[k]);
         if (lane == 0) wsum[warp][k] = v;
     }
+    if constexpr (kLow) {
+        low = warp_sum(low);
+        if (lane == 0) wlow[warp] = low;
+    }
     if (__syncthreads_or(odd)) {
         if (!odd)
             for (int k = 0; k < 5; k++) sh[k][threadIdx.x] = Acc{0.0, 0.0};
@@ -255,6 +292,11 @@ __global__ void __launch_bounds__(kBlock, 2) k_reduce(LatDesc d, int layout, Red
         for (int w = 0; w < kBlock / 32; w++) v += wsum[w][threadIdx.x];
         partial[blockIdx.x].fix[threadIdx.x] = layout && threadIdx.x >= 1 && threadIdx.x <= 3 ? -v : v;
         partial[blockIdx.x].acc[threadIdx.x] = sh[threadIdx.x][0];
+    } else if (threadIdx.x == 5) {
+        uint64_t v = 0;
+        if (kLow)
+            for (int w = 0; w < kBlock / 32; w++) v += wlow[w];
+        partial[blockIdx.x].low = v;
     }
 }
 
@@ -264,20 +306,24 @@ __global__ void __launch_bounds__(160) k_reduce_final(const RedPartial *partial,
                                                       double *out) {
     const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
     i128 v = 0;
+    uint64_t low = 0;
     Acc a{0.0, 0.0};
 #pragma unroll 4
     for (int b = lane; b < nblocks; b += 32) {
         v += partial[b].fix[q];
+        if (q == 4) low += partial[b].low;
         const Acc o = partial[b].acc[q];
         if (!(o.s == 0.0 && o.c == 0.0)) a.merge(o);
     }
     v = warp_sum(v);
+    low = warp_sum(low);
+    v += (i128)(low >> 32);
     for (int o = 16; o > 0; o >>= 1) {
         const Acc other{__shfl_down_sync(0xffffffffu, a.s, o), __shfl_down_sync(0xffffffffu, a.c, o)};
         if (lane + o < 32) a.merge(other);
     }
     if (lane == 0) {
-        a.add(q == 4 ? 0.5 * to_double(v, lsb_e) : to_double(v, lsb));
+        a.add(q == 4 ? 0.5 * to_double(v, lsb_e, (uint32_t)low) : to_double(v, lsb));
         out[q] = a.s + a.c;
     }
 }
@@ -285,10 +331,12 @@ __global__ void __launch_bounds__(160) k_reduce_final(const RedPartial *partial,
 // Velocity difference of two lattices of the same size over the fluid cells
 // of `a`: max |ua - ub|, sum |ua - ub|^2, sum |ub|^2, max |ub|, cell count,
 // with u the momentum of the stored populations in the given slot layouts.
-// Momenta in units of 2^-61, squares of 2^-122, their sums of 2^-90.
+// Momenta in units of 2^-61, squares of 2^-122, their sums of 2^-90 and the
+// lower words' (Squares).
 struct CmpPartial {
     i128 fix[4];  // max |ua - ub|^2, its sum, sum |ub|^2, max |ub|^2
     double acc[4];  // the same of cells outside the fixed-point bounds: max, sum, sum, max
+    uint64_t low[2];  // lower words of the two sums
     double cells;
     double pad;
 };
@@ -300,7 +348,10 @@ __global__ void __launch_bounds__(kBlock, 2) k_compare(LatDesc a, int la, LatDes
     using RB = typename Store<SB>::R;
     __shared__ double sh[4][kBlock];
     __shared__ i128 wred[kBlock / 32][5];
-    i128 mx = 0, se = 0, sr = 0, mr = 0;
+    __shared__ uint64_t wlow[kBlock / 32][2];
+    i128 mx = 0, mr = 0;
+    Squares<sizeof(RA) == 8 || sizeof(RB) == 8> se;
+    Squares<sizeof(RB) == 8> sr;
     uint32_t cnt = 0;
     double dv[4] = {0.0, 0.0, 0.0, 0.0};
     bool odd = false;
@@ -326,8 +377,8 @@ __global__ void __launch_bounds__(kBlock, 2) k_compare(LatDesc a, int la, LatDes
             }
             mx = (i128)e2 > mx ? (i128)e2 : mx;
             mr = (i128)r2 > mr ? (i128)r2 : mr;
-            se += (i128)(e2 >> 32);
-            sr += (i128)(r2 >> 32);
+            se.add(e2);
+            sr.add(r2);
         } else {
             odd = true;
             double r, ua[3], ub[3];
@@ -347,12 +398,15 @@ __global__ void __launch_bounds__(kBlock, 2) k_compare(LatDesc a, int la, LatDes
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     mx = warp_max(mx);
-    se = warp_sum(se);
-    sr = warp_sum(sr);
+    se.hi = warp_sum(se.hi);
+    sr.hi = warp_sum(sr.hi);
+    se.lo = warp_sum(se.lo);
+    sr.lo = warp_sum(sr.lo);
     mr = warp_max(mr);
     const i128 n = warp_sum((i128)cnt);
     if (lane == 0) {
-        wred[warp][0] = mx; wred[warp][1] = se; wred[warp][2] = sr; wred[warp][3] = mr; wred[warp][4] = n;
+        wred[warp][0] = mx; wred[warp][1] = se.hi; wred[warp][2] = sr.hi; wred[warp][3] = mr; wred[warp][4] = n;
+        wlow[warp][0] = se.lo; wlow[warp][1] = sr.lo;
     }
     if (__syncthreads_or(odd)) {
         for (int k = 0; k < 4; k++) sh[k][threadIdx.x] = dv[k];
@@ -383,6 +437,11 @@ __global__ void __launch_bounds__(kBlock, 2) k_compare(LatDesc a, int la, LatDes
         } else {
             p.cells = (double)(int64_t)v;
         }
+    } else if (threadIdx.x < 7) {
+        const int k = threadIdx.x - 5;
+        uint64_t v = 0;
+        for (int w = 0; w < kBlock / 32; w++) v += wlow[w][k];
+        partial[blockIdx.x].low[k] = v;
     }
 }
 
@@ -390,8 +449,10 @@ __global__ void __launch_bounds__(160) k_compare_final(const CmpPartial *partial
     const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool is_max = q == 0 || q == 3;
     i128 v = 0;
+    uint64_t low = 0;
     double a = 0.0;
     for (int b = lane; b < nblocks; b += 32) {
+        if (q == 1 || q == 2) low += partial[b].low[q - 1];
         const i128 o = q < 4 ? partial[b].fix[q] : (i128)0;
         const double s = q < 4 ? partial[b].acc[q] : partial[b].cells;
         if (is_max) {
@@ -403,11 +464,13 @@ __global__ void __launch_bounds__(160) k_compare_final(const CmpPartial *partial
         }
     }
     v = is_max ? warp_max(v) : warp_sum(v);
+    low = warp_sum(low);
+    v += (i128)(low >> 32);
     for (int o = 16; o > 0; o >>= 1) {
         const double s = __shfl_down_sync(0xffffffffu, a, o);
         if (lane + o < 32) a = is_max ? fmax(a, s) : a + s;
     }
-    if (lane == 0) out[q] = is_max ? fmax(a, sqrt(to_double(v, 122))) : a + to_double(v, 90);
+    if (lane == 0) out[q] = is_max ? fmax(a, sqrt(to_double(v, 122))) : a + to_double(v, 90, (uint32_t)low);
 }
 
 int red_blocks(const LatDesc &d, int per_thread) {
