@@ -84,6 +84,7 @@ void set_params_desc(LatDesc &h, int storage, const lbm_params &p) {
         for (int i = 0; i < P_COUNT; i++) h.pd[i] = (double)h.pf[i];
     }
     h.grav = grav;
+    h.not_fix64 = fx_params(h.pd[P_INV_TAU], h.pd[P_TAU0], h.pd[P_LES]) ? 0 : 1;
     h.gmode = p.gravity_mode ? 1 : 0;
 }
 

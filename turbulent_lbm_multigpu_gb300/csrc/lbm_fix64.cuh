@@ -319,8 +319,18 @@ LBM_HD double fx_sqrt(double x) {
     return hi32(bits_of(x)) - 0x38700000u < 0x0DC00000u ? sqrt_int(x) : sqrt(x);  // [2^-120, 2^100)
 }
 
-// The collision of an ordinary fluid cell from its moments on the grid
-// (operation by operation that of collide()): populations x in, f out; vx,
+// Whether the parameters are ones fx_collide reproduces for every ordinary
+// cell: a finite rate, and with the subgrid model a coefficient and a tau0
+// whose sum of roots stays within rcp_int's range (the strain norm q of
+// ordinary populations is below 2^5).  Others (negative, huge, infinite, not a
+// number) take the double arithmetic.
+LBM_HD bool fx_params(double inv_tau, double tau0, double les_c) {
+    if (les_c == 0.0) return inv_tau - inv_tau == 0.0;
+    return les_c > 0.0 && les_c <= 0x1p100 && tau0 >= 0.5 && tau0 <= 0x1p50;
+}
+
+// The collision of an ordinary fluid cell from its moments on the grid, under
+// parameters that fx_params accepts (operation by operation that of collide()): populations x in, f out; vx,
 // vy, vz and dp come out as doubles.
 template <bool LES>
 LBM_HD void fx_collide(const Fx x[19], Fx r, Fx jx, Fx jy, Fx jz, double inv_tau, double tau0, double les_c, double f[19],
