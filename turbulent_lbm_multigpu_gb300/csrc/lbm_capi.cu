@@ -1130,9 +1130,10 @@ int domain_record(lbm_domain *D, cudaStream_t st, cudaEvent_t *out) {
     return 0;
 }
 
-// dep: programmatic dependence on the launch before (a lone lattice's steps
-// launched one by one; with exchange launches in between, or captured into a
-// graph, it costs: half 128x120x110 in 2x2x1 subdomains 32.9 -> 41.9 us a step).
+// dep: programmatic dependence on the launch before (a lone lattice's steps).
+// With exchange launches in between, captured, it gains nothing (2x2x1
+// subdomains, us per step without / with: half 128x120x110 32.6 / 32.8, float
+// 256^3 431.1 / 431.4; float 100^3 in 2x2x2 28.7 / 28.1, c16 27.7 / 28.3).
 int domain_one_step(lbm_domain *D, int parity, cudaStream_t st, bool store, bool timed, Dep dep) {
     const bool les = uses_les(D->subs[0]->h);
     const int sv = store ? D->store_v : 0, sr = store ? D->store_rho : 0;
@@ -1428,7 +1429,7 @@ int lbm_cu_domain_run(lbm_domain *D, int steps, int use_graph, void *stream) {
     int pairs = (steps - done) / 2;
     if (D->store_interval == 0 && (steps - done) % 2 == 0 && pairs > 0) pairs--;  // last pair stores
     // a lone subdomain's steps follow one another faster launched one by one
-    // with programmatic dependence (float 24^3 4.1 -> 3.5 us, 64^3 8.2 -> 6.9,
+    // with programmatic dependence (float 24^3 4.1 -> 2.8 us, 64^3 8.2 -> 6.6,
     // 128^3 54.2 -> 53.1; half 64^3 7.2 -> 6.2)
     if (pairs > 0 && use_graph && plain_pairs && !D->profile && D->subs.size() > 1) {
         if (!D->graph) {

@@ -24,12 +24,14 @@ int fail(const std::string &m);
 
 inline cudaStream_t S(void *s) { return (cudaStream_t)s; }
 
-// Launch of a kernel that begins with follow_previous_grid(): its blocks may
-// be set up while the grid before it on the stream drains.  Measured on runs
-// launched step by step (us per step, plain -> this): float 24^3 5.17 -> 3.48,
-// 64^3 9.20 -> 6.90, 128^3 54.9 -> 53.1, 256^3 398.6 -> 396.1; half 24^3
-// 6.71 -> 4.94, 128^3 31.9 -> 30.5: about 2 us a launch.  Not for captured
-// graphs or steps with exchange launches between them (domain_one_step).
+// Launch of a kernel that begins with follow_previous_grid(): its blocks are
+// set up before the grid before it on the stream has written back its results.
+// Measured on runs launched step by step (us per step, plain -> this): float
+// 24^3 5.12 -> 2.83, 64^3 9.22 -> 6.64, 128^3 55.6 -> 52.6; half 24^3 5.12 ->
+// 2.64, 128^3 33.0 -> 30.3; double 64^3 56.9 -> 54.5: about 2.5 us a launch.
+// Also faster in a graph that a caller captures (float 64^3 6.84 -> 6.41) and
+// between lbm_cu_halo copies (four 64^3 lattices, step and exchange: 71.0 ->
+// 60.1 us).  Not used for the steps of several subdomains (domain_one_step).
 struct Dep {
     bool on = true;  // false: an ordinary launch
 };
