@@ -372,9 +372,10 @@ lbm_lattice *lbm_cu_batch_lattice(lbm_batch *b, int index);
  * HBM budget (and fewer than max_active run), advances every running solve
  * by up to max_steps steps in shared launches (stopping when the first one
  * completes), and retires completed solves, whose fields stay resident
- * until released.  A released solve's device memory is kept for later ones,
- * at most an eighth of the budget (all of it within the budget), and freed
- * with the server.  A solve's result does not depend on what else runs. */
+ * until released.  A released solve's device memory is kept for later ones
+ * of the same size, at most an eighth of the budget (all of it within the
+ * budget, not counted in hbm_used), until a tick finds nothing to run or the
+ * server is destroyed.  A solve's result does not depend on what else runs. */
 int lbm_cu_server_create(double hbm_budget_bytes, int max_active, int store_velocity, lbm_server **out);
 int lbm_cu_server_destroy(lbm_server *s);
 /* As lbm_cu_batch_set_kernel_shape; a server starts with shape 3. */

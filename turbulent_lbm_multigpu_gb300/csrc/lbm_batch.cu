@@ -348,8 +348,11 @@ struct lbm_server {
     // Device blocks, one per resident solve.  A released solve's block is
     // kept for a later one, at most an eighth of the budget of them and all
     // of them within it (cudaMalloc and cudaFree of a solve's fields took a
-    // tenth of a burst's time).  The device has finished with a block when it
-    // changes hands (release); the server frees them when it is destroyed.
+    // tenth of a burst's time).  No block is larger than its solve's share of
+    // the budget (cavity_bytes), so that solves are admitted by `used` alone.
+    // The device has finished with a block when it changes hands (release).
+    // A tick that finds nothing to run gives the idle ones back (server_tick),
+    // and so does the server's end.
     struct Block {
         void *p;
         size_t bytes;
@@ -371,13 +374,13 @@ struct lbm_server {
         idle_bytes -= (double)idle[i].bytes;
         idle.erase(idle.begin() + i);
     }
-    // A block of at least `bytes`: the smallest idle one that is no more than
-    // a quarter larger and fits the budget, else a new one.
-    int take(size_t bytes, Block *out) {
+    // A block of `bytes` to `most` bytes: the smallest such idle one, else a
+    // new one of `bytes`.
+    int take(size_t bytes, size_t most, Block *out) {
         size_t best = idle.size();
         for (size_t i = 0; i < idle.size(); i++)
-            if (idle[i].bytes >= bytes && idle[i].bytes <= bytes + bytes / 4 &&
-                held - idle_bytes + (double)idle[i].bytes <= budget && (best == idle.size() || idle[i].bytes < idle[best].bytes))
+            if (idle[i].bytes >= bytes && idle[i].bytes <= most &&
+                (best == idle.size() || idle[i].bytes < idle[best].bytes))
                 best = i;
         if (best < idle.size()) {
             *out = idle[best];
@@ -593,16 +596,15 @@ static int server_admit(lbm_server *s, cudaStream_t st) {
     int admitted = 0;
     while (!s->queue.empty()) {
         const lbm_server::Pending &p = s->queue.front();
-        const double need = (double)cavity_bytes(p.spec, s->e.store_v);
-        const size_t bytes = lattice_block_bytes(p.spec.nx, p.spec.ny, p.spec.nz, p.spec.storage, s->e.store_v);
-        if (s->used + need > s->budget || s->held - s->idle_bytes + (double)bytes > s->budget ||
-            s->e.active_count() >= s->max_active)
-            break;
+        const size_t share = cavity_bytes(p.spec, s->e.store_v);
+        const double need = (double)share;
+        if (s->used + need > s->budget || s->e.active_count() >= s->max_active) break;
         Ensemble::Slot slot;
         slot.spec = p.spec;
         slot.id = p.id;
         lbm_server::Block blk{};
-        if (s->take(bytes, &blk)) return -1;
+        const size_t bytes = lattice_block_bytes(p.spec.nx, p.spec.ny, p.spec.nz, p.spec.storage, s->e.store_v);
+        if (s->take(bytes, share, &blk)) return -1;
         const lbm_params prm = cavity_params(p.spec);
         if (lattice_in_block(p.spec.nx, p.spec.ny, p.spec.nz, p.spec.storage, s->e.store_v, blk.p, &slot.lat) ||
             lbm_cu_set_params(slot.lat, &prm) || cavity_reset(slot.lat, p.spec, st)) {
@@ -635,6 +637,8 @@ int lbm_cu_server_tick(lbm_server *s, int64_t max_steps, int use_graph, int *adm
     const int adm = server_admit(s, st);
     if (adm < 0) return -1;
     if (admitted) *admitted = adm;
+    if (s->queue.empty() && s->e.active_count() == 0)
+        while (!s->idle.empty()) s->drop_idle(0);
     const int64_t k = std::min(max_steps > 0 ? max_steps : INT64_MAX, s->e.min_remaining());
     if (k > 0) {
         int64_t cells = 0;
