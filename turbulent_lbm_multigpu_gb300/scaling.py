@@ -65,7 +65,7 @@ def _params(api, storage, length):
 
 
 def run_one(api, size, nums, storage, steps, warmup=10):
-    """Seconds for `steps` steps of the domain (CUDA graph replay, synchronised)."""
+    """Seconds for `steps` steps of the domain (graph replay of several subdomains, synchronised)."""
     D = api.Domain(size, nums, storage, store_velocity=False, store_density=False)
     D.set_params(_params(api, storage, size[0]))
     D.set_halo_mode(1)
