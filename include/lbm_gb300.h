@@ -355,8 +355,9 @@ int lbm_cu_batch_reset(lbm_batch *b, void *stream);
 /* Ensemble kernel shape: 1 one cell per thread (default), 2 two cells per
  * thread (cavities with even nx), 3 as 1 but the cavities of a 16-bit storage
  * type run the staged tiles when every member of a launch is at the same kind
- * of step and it is as large as shape 0 of a lattice asks for.  Results are
- * the same for every shape. */
+ * of step and the unfinished cavities of that type together are as large as
+ * shape 0 of a lattice asks for (rows of any one that are not a multiple of 8
+ * count for all).  Results are the same for every shape. */
 int lbm_cu_batch_set_kernel_shape(lbm_batch *b, int cells_per_thread);
 /* Autotuner: times `trial_steps` steps of the whole ensemble for each kernel
  * shape (1, 2, 3), keeps the fastest, and resets. */

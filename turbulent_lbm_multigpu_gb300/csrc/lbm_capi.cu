@@ -482,12 +482,11 @@ static int launch_staged_batch_t(bool beta, bool les, const BatchArgs &a, int ti
 
 int launch_staged_batch(int storage, bool beta, bool les, const BatchArgs &a, int tiles, Dep dep, cudaStream_t st) {
     switch (storage) {
-        case kF32: return launch_staged_batch_t<float>(beta, les, a, tiles, dep, st);
         case kF16: return launch_staged_batch_t<__half>(beta, les, a, tiles, dep, st);
         case kBF16: return launch_staged_batch_t<__nv_bfloat16>(beta, les, a, tiles, dep, st);
         case kC16: return launch_staged_batch_t<c16_t>(beta, les, a, tiles, dep, st);
     }
-    return fail("the staged kernels take float, half or bfloat16 storage");
+    return fail("the staged ensemble kernels take the 16-bit storage types");
 }
 
 int launch_step(int storage, int shape, int parity, bool les, const LatDesc *htab, int ntab, int sv, int sr,

@@ -13,9 +13,10 @@
 // addition followed by rounding to 53 significant bits, half to even: about
 // ten integer operations (Fx).  Moments, pair sums, equilibria (their
 // constants 1/18, 1/36, 1/3 are 24-bit floats, so the products need 88 bits)
-// and the differences feq - f run that way; products of two velocities, the
-// subgrid model's square roots and the relaxation's product and sum stay on
-// the FP64 pipe, which works beside the integer ones.
+// and the differences feq - f run that way, the subgrid model's square roots
+// and reciprocal in integers of their own; products of two velocities, the
+// strain norm and the relaxation's product and sum stay on the FP64 pipe,
+// which works beside the integer ones.
 //
 // Measured (256^3 in 2x2x1 subdomains, subgrid model, per step): 8.39 ms ->
 // 3.00 ms (2.00k -> 5.60k MLUPS), 76 double operations per cell instead of

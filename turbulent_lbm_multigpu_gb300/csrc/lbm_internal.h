@@ -83,7 +83,9 @@ inline int cells_per_block(bool pair) { return pair ? kPairCells : kBlock; }
 // not whole 16-byte units: 121x99x87 (1.04 M) 17.4 / 18.3, 129x128x128 33.7 /
 // 32.2 (its beta kernels 41.3 / 41.8), 177x176x176 102.5 / 77.9; c16 64^3 6.76 / 8.69, 112^3 26.9 / 26.9,
 // 176^3 111 / 92.9.  The alpha kernels alone cross earlier (half, us): 64^3
-// 10.5 / 10.7, 96^3 18.6 / 17.5, 121x99x87 20.7 / 18.8.
+// 10.5 / 10.7, 96^3 18.6 / 17.5, 121x99x87 20.7 / 18.8.  The lines are cell
+// counts where this GPU's two kernels cross, not multiples of its resident
+// blocks.
 constexpr int64_t kStagedAlphaCells = 786432;    // alpha steps
 constexpr int64_t kStagedCells = 1310720;        // beta steps, every row whole 16-byte units
 constexpr int64_t kStagedRaggedCells = 2359296;  // beta steps, other rows
@@ -120,10 +122,9 @@ int launch_step(int storage, int shape, int parity, bool les, const LatDesc *hta
 int step_lattice(const lbm_lattice *l, int parity, bool store, cudaStream_t st);
 // Cells per staged tile of a storage type (0: not staged).
 int staged_cells(int storage);
-// One step of up to kBatchLattices lattices, all at an alpha step or all at
-// a beta step, through the staged tiles (first_block / nblocks of the
-// descriptors count tiles of staged_cells; a beta step needs every nx a
-// multiple of 16 bytes of populations).
+// One step of up to kBatchLattices 16-bit lattices of any row length, all at
+// an alpha step or all at a beta step, through the staged tiles (first_block /
+// nblocks of the descriptors count tiles of staged_cells).
 int launch_staged_batch(int storage, bool beta, bool les, const BatchArgs &a, int tiles, Dep dep, cudaStream_t st);
 // One lattice block of a checkpoint file (lbm_io.cu).
 int ckpt_write_lattice(FILE *f, lbm_lattice *l, int64_t counter);
