@@ -22,8 +22,8 @@
 // 3.00 ms (2.00k -> 5.60k MLUPS), 76 double operations per cell instead of
 // 275; the FP64 pipe is 65 % busy, the shift and logic pipe 72 %, so that
 // neither side has much left to take from the other (the last addition of 4
-// to 12 populations moved over here too: 3.08-3.18 ms); 48x40x36 43 -> 21 us,
-// 24^3 24 -> 17 us.
+// to 12 populations moved over here too: 3.08-3.18 ms); 48x40x36 45 -> 19 us,
+// 24^3 25 -> 15 us.
 //
 // Every step rounds as the double operation it stands for, so the results
 // are the same bits.  Cells outside the range (populations outside
@@ -460,9 +460,9 @@ LBM_HD void fx_lid(double lid, double f[19], double &dp) {
 // exact, products are cut at 2^-61 (a double population's last place is
 // 2^-57 to 2^-59), and only the new population rounds to 53 bits.  About 10
 // double operations per cell remain, in the strain norm.  Measured (256^3 in
-// 2x2x1 subdomains, subgrid model): 6.14 -> 1.68 ms per step (9.99k MLUPS) at
+// 2x2x1 subdomains, subgrid model): 6.14 -> 1.64 ms per step (10.2k MLUPS) at
 // 2 blocks of 256 per SM (128 registers; 3 blocks spill more and take 1.86,
-// 4 blocks 2.55), 1,950-2,100 instructions per cell, the shift and logic pipe
+// 4 blocks 2.55), 1,940-2,000 instructions per cell, the shift and logic pipe
 // 60 % busy.
 
 // High half of the signed 128-bit product.
